@@ -458,7 +458,8 @@ attention_decode_tiled_kernel(const Params p) {
 // query fragments stay in registers for the whole launch, and no warp keeps output accumulators that others share:
 //   S = Q K^T   warp = (16-row tile mt, slice of the tile's timesteps).  The contraction index is permuted so that a lane's
 //               operands are sixteen consecutive bytes of a row; A = Q (registers), B = K^T.
-//   softmax     row maxima of the slices meet in shared memory; probabilities go there in 16 bits, row-major.
+//   softmax     row maxima of the slices meet in shared memory; probabilities go there in 16 bits, row-major, each slice's
+//               relative to a reference of its own: its maximum, unless that lies far below the running one (kOwnReference).
 //   O += P V    warp = 32 dims of every row over all timesteps of the tile: A = P (ldmatrix), B = V, a lane pairing the
 //               bytes of neighbouring timesteps; column c of n-tile j is dim 32 warp + 4 c + j, so a lane ends up with
 //               eight consecutive dims of its rows and stores them as they are.
@@ -466,6 +467,12 @@ attention_decode_tiled_kernel(const Params p) {
 // multiplied; three block barriers per tile.  Per 64 FP8 rows and two row tiles: 116 KB through the shared-memory port.
 // The bytes 0x7F / 0xFF (never written by the append) convert to NaN where the reference reads +-448: a NaN anywhere in
 // the CTA's state sends it through a second pass that rewrites them first (FIX).
+// Why the slices keep references of their own: the largest weight of each is then exactly one, and how much the rounding of
+// the weights costs is decided by the few largest.  With one reference per tile the float32 partials were further from
+// float64 than those of the ldmatrix kernel, whose warps keep a maximum each: BF16 1.3 - 2.8 times (flat attention: the
+// outputs 4 - 7 %), now 0.2 - 1.06 times; FP8 1.2 - 2.7 times, now 0.6 - 1.9 (outputs within 0.2 %).  Two 16-bit terms per
+// weight leave a hundredth of that error and cost a quarter of the time.
+// FP8 probabilities carry a factor 2^15 (float16 holds 65504), so that those far below the reference keep their bits.
 // Measured figures are at launch_verify.
 template <bool FP8> struct VerifyTile {
   static constexpr uint32_t kRowBytes = FP8 ? kD : 2u * kD;
@@ -474,9 +481,16 @@ template <bool FP8> struct VerifyTile {
   static constexpr uint32_t kPStride = kRows + 8u;                  // 16-bit elements per row of probabilities
 };
 constexpr uint32_t kVerifyThreads = 256, kVerifyWarps = kVerifyThreads / 32, kVerifyStages = 3;
+constexpr float kVerifyPScale = 32768.f;
+constexpr float kVerifyLog2 = 0.0625f * 1.4426950408889634f;         // rsqrt(256) * log2(e): scores to powers of two
+constexpr float kOwnReference = 4.0f / kVerifyLog2;                  // a slice whose largest weight is 2^-4 or more
 template <bool FP8, int MT> constexpr uint32_t verify_smem_bytes() {
   return kVerifyStages * 2u * VerifyTile<FP8>::kHalf + 16u * MT * VerifyTile<FP8>::kPStride * 2u +
-         (kVerifyWarps / MT + 1u) * 16u * MT * 4u;
+         2u * (kVerifyWarps / MT) * 16u * MT * 4u;
+}
+// factor that takes sums relative to reference `from` to reference `to` (from = -inf: nothing has been summed yet)
+__device__ __forceinline__ float verify_rescale(float from, float to) {
+  return from == -INFINITY ? 1.f : exp2f((from - to) * kVerifyLog2);
 }
 
 __device__ __forceinline__ uint32_t bytes_nan_to_448(uint32_t w) {
@@ -491,23 +505,24 @@ __device__ __forceinline__ void e4m3x4_to_f16(uint32_t w, uint32_t &lo, uint32_t
 
 template <bool FP8, int MT, bool FIX>
 __device__ __forceinline__ void verify_pass(const Params &p, uint8_t *smem, const uint32_t (&qf)[16][4], float (&o)[MT][4][4],
-                                            float &m_lo, float &m_hi, float &l_lo, float &l_hi, uint32_t t0, uint32_t t1,
-                                            uint32_t start, uint32_t lim_lo, uint32_t lim_hi, uint32_t kvh) {
+                                            float &m_lo, float &m_hi, float &l_lo, float &l_hi, float &ref_lo, float &ref_hi,
+                                            uint32_t t0, uint32_t t1, uint32_t start, uint32_t lim_lo, uint32_t lim_hi, uint32_t kvh) {
   using VT = VerifyTile<FP8>;
   constexpr uint32_t RB = VT::kRowBytes, T = VT::kRows, TS = kVerifyWarps / MT, W = T / TS, CH = RB / 16u, PS = VT::kPStride;
-  constexpr float kScaleLog2 = 0.0625f * 1.4426950408889634f;        // rsqrt(256) * log2(e)
+  // slices that share a reference (an MMA spans 16 timesteps), references per tile, MMA steps per reference
+  constexpr uint32_t SP = W < 16u ? 16u / W : 1u, RS = TS / SP, KS = SP * W / 16u;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, g = lane >> 2, t = lane & 3u;
   const uint32_t mt = warp % MT, th = warp / MT;
   const uint32_t ring = smem_u32(smem);
   uint16_t *sp = reinterpret_cast<uint16_t *>(smem + kVerifyStages * 2u * VT::kHalf);          // [16 MT][PS]
   float *smax = reinterpret_cast<float *>(sp + 16u * MT * PS);       // [TS][16 MT]
-  float *scorr = smax + TS * 16u * MT;                               // [16 MT]
+  float *scorr = smax + TS * 16u * MT;                               // [RS][16 MT]: rescale of the outputs ahead of slice h
   const uint32_t n_tiles = t1 > t0 ? (t1 - t0 + T - 1u) / T : 0u;
 #pragma unroll
   for (int a = 0; a < MT; ++a)
 #pragma unroll
     for (int j = 0; j < 4; ++j) o[a][j][0] = o[a][j][1] = o[a][j][2] = o[a][j][3] = 0.f;
-  m_lo = m_hi = -INFINITY;
+  m_lo = m_hi = ref_lo = ref_hi = -INFINITY;                         // ref: the reference of the outputs as they stand
   l_lo = l_hi = 0.f;
 
   // K chunk c of row r at c ^ 4 (r & 1), V chunk c of row r at c ^ 2 ((r / 2) & 3): fragment reads free of bank conflicts
@@ -589,54 +604,72 @@ __device__ __forceinline__ void verify_pass(const Params &p, uint8_t *smem, cons
       smax[th * 16u * MT + r_hi] = mx_hi;
     }
     __syncthreads();
-    float mn_lo = m_lo, mn_hi = m_hi;
+    float mn_lo = m_lo, mn_hi = m_hi, top_lo[RS], top_hi[RS];
 #pragma unroll
-    for (uint32_t h = 0; h < TS; ++h) {
-      mn_lo = fmaxf(mn_lo, smax[h * 16u * MT + r_lo]);
-      mn_hi = fmaxf(mn_hi, smax[h * 16u * MT + r_hi]);
+    for (uint32_t h = 0; h < RS; ++h) {
+      top_lo[h] = smax[h * SP * 16u * MT + r_lo];
+      top_hi[h] = smax[h * SP * 16u * MT + r_hi];
+#pragma unroll
+      for (uint32_t i = 1; i < SP; ++i) {
+        top_lo[h] = fmaxf(top_lo[h], smax[(h * SP + i) * 16u * MT + r_lo]);
+        top_hi[h] = fmaxf(top_hi[h], smax[(h * SP + i) * 16u * MT + r_hi]);
+      }
+      mn_lo = fmaxf(mn_lo, top_lo[h]);
+      mn_hi = fmaxf(mn_hi, top_hi[h]);
     }
-    const float al_lo = m_lo == -INFINITY ? (mn_lo == -INFINITY ? 1.f : 0.f) : exp2f((m_lo - mn_lo) * kScaleLog2);
-    const float al_hi = m_hi == -INFINITY ? (mn_hi == -INFINITY ? 1.f : 0.f) : exp2f((m_hi - mn_hi) * kScaleLog2);
-    const float ref_lo = mn_lo == -INFINITY ? 0.f : mn_lo, ref_hi = mn_hi == -INFINITY ? 0.f : mn_hi;
+    l_lo *= verify_rescale(m_lo, mn_lo);                             // l is relative to the running maximum
+    l_hi *= verify_rescale(m_hi, mn_hi);
     m_lo = mn_lo;
     m_hi = mn_hi;
+    float before_lo = ref_lo, before_hi = ref_hi, own_lo = 0.f, own_hi = 0.f;
+#pragma unroll
+    for (uint32_t h = 0; h < RS; ++h) {
+      const float now_lo = top_lo[h] >= m_lo - kOwnReference ? top_lo[h] : m_lo;
+      const float now_hi = top_hi[h] >= m_hi - kOwnReference ? top_hi[h] : m_hi;
+      if (h == th / SP) {
+        before_lo = ref_lo; before_hi = ref_hi;
+        own_lo = now_lo; own_hi = now_hi;
+      }
+      ref_lo = now_lo; ref_hi = now_hi;
+    }
+    if (th % SP == 0u && t == 0u) {
+      scorr[(th / SP) * 16u * MT + r_lo] = verify_rescale(before_lo, own_lo);
+      scorr[(th / SP) * 16u * MT + r_hi] = verify_rescale(before_hi, own_hi);
+    }
+    const float from_lo = own_lo == -INFINITY ? 0.f : own_lo, from_hi = own_hi == -INFINITY ? 0.f : own_hi;
     float sum_lo = 0.f, sum_hi = 0.f;
 #pragma unroll
     for (uint32_t nb = 0; nb < W / 8u; ++nb) {
-      const float p0 = exp2f((s[nb][0] - ref_lo) * kScaleLog2), p1 = exp2f((s[nb][1] - ref_lo) * kScaleLog2);
-      const float p2 = exp2f((s[nb][2] - ref_hi) * kScaleLog2), p3 = exp2f((s[nb][3] - ref_hi) * kScaleLog2);
+      float p0 = exp2f((s[nb][0] - from_lo) * kVerifyLog2), p1 = exp2f((s[nb][1] - from_lo) * kVerifyLog2);
+      float p2 = exp2f((s[nb][2] - from_hi) * kVerifyLog2), p3 = exp2f((s[nb][3] - from_hi) * kVerifyLog2);
       sum_lo += p0 + p1;
       sum_hi += p2 + p3;
+      if (FP8) { p0 *= kVerifyPScale; p1 *= kVerifyPScale; p2 *= kVerifyPScale; p3 *= kVerifyPScale; }
       const uint32_t at = th * W + 8u * nb + 2u * t;
       *reinterpret_cast<uint32_t *>(sp + r_lo * PS + at) = pack2<FP8>(p0, p1);
       *reinterpret_cast<uint32_t *>(sp + r_hi * PS + at) = pack2<FP8>(p2, p3);
     }
-    l_lo = l_lo * al_lo + sum_lo;                                    // this lane's timesteps only; the lanes meet after the loop
-    l_hi = l_hi * al_hi + sum_hi;
-    if (th == 0u && t == 0u) { scorr[r_lo] = al_lo; scorr[r_hi] = al_hi; }
+    l_lo += sum_lo * verify_rescale(own_lo, m_lo);                   // this lane's timesteps only; the lanes meet after the loop
+    l_hi += sum_hi * verify_rescale(own_hi, m_hi);
     __syncthreads();
 
     // ---- O += P V, dims 32 warp .. + 31 of every row
-    float c_lo[MT], c_hi[MT];
-    bool moved = false;
-#pragma unroll
-    for (int a = 0; a < MT; ++a) {
-      c_lo[a] = scorr[16 * a + g];
-      c_hi[a] = scorr[16 * a + g + 8u];
-      moved |= c_lo[a] != 1.f || c_hi[a] != 1.f;
-    }
-    if (__any_sync(0xffffffffu, moved)) {                            // a running maximum moved (rare after the first tiles)
-#pragma unroll
-      for (int a = 0; a < MT; ++a)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          o[a][j][0] *= c_lo[a]; o[a][j][1] *= c_lo[a];
-          o[a][j][2] *= c_hi[a]; o[a][j][3] *= c_hi[a];
-        }
-    }
     const uint32_t p_addr = smem_u32(sp) + ((lane & 15u) * PS + 8u * (lane >> 4)) * 2u;
-#pragma unroll 2
+    // (all steps unrolled and no test for factors of one: loads and conversions of V run ahead of the multiplications; BF16, 16
+    // tokens, context 32768: 84.2 -> 77.0 us)
+#pragma unroll
     for (uint32_t ks = 0; ks < T / 16u; ++ks) {
+      if (ks % KS == 0u) {                                           // the next slice: outputs to its reference
+#pragma unroll
+        for (int a = 0; a < MT; ++a) {
+          const float c_lo = scorr[ks / KS * 16u * MT + 16 * a + g], c_hi = scorr[ks / KS * 16u * MT + 16 * a + g + 8u];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            o[a][j][0] *= c_lo; o[a][j][1] *= c_lo;
+            o[a][j][2] *= c_hi; o[a][j][3] *= c_hi;
+          }
+        }
+      }
       const uint8_t *vt = sv + (ks * 16u + 2u * t) * RB;
       uint32_t b0[4], b1[4];
       if (FP8) {
@@ -670,7 +703,7 @@ __device__ __forceinline__ void verify_pass(const Params &p, uint8_t *smem, cons
 }
 
 template <bool FP8, int MT>
-__global__ void __launch_bounds__(kVerifyThreads, 1)
+__global__ void __maxnreg__(MT <= 2 ? 192 : 255)       // one or two row tiles: a CTA of the reduce finds its registers beside it
 attention_verify_kernel(const Params p) {
   using VT = VerifyTile<FP8>;
   constexpr uint32_t TS = kVerifyWarps / MT;
@@ -720,8 +753,8 @@ attention_verify_kernel(const Params p) {
     }
   }
 
-  float o[MT][4][4], m_lo, m_hi, l_lo, l_hi;
-  verify_pass<FP8, MT, false>(p, smem, qf, o, m_lo, m_hi, l_lo, l_hi, t0, t1, start, lim_lo, lim_hi, kvh);
+  float o[MT][4][4], m_lo, m_hi, l_lo, l_hi, ref_lo, ref_hi;
+  verify_pass<FP8, MT, false>(p, smem, qf, o, m_lo, m_hi, l_lo, l_hi, ref_lo, ref_hi, t0, t1, start, lim_lo, lim_hi, kvh);
   if (FP8) {
     float probe = l_lo + l_hi;
 #pragma unroll
@@ -729,19 +762,24 @@ attention_verify_kernel(const Params p) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) probe += (o[a][j][0] + o[a][j][1]) + (o[a][j][2] + o[a][j][3]);
     if (__syncthreads_or(probe != probe))
-      verify_pass<FP8, MT, true>(p, smem, qf, o, m_lo, m_hi, l_lo, l_hi, t0, t1, start, lim_lo, lim_hi, kvh);
+      verify_pass<FP8, MT, true>(p, smem, qf, o, m_lo, m_hi, l_lo, l_hi, ref_lo, ref_hi, t0, t1, start, lim_lo, lim_hi, kvh);
   }
 
-  // ---- partials: l of the slices meets in shared memory, outputs go out as they are
+  // ---- partials: l of the slices and the outputs' last step, to the running maximum, meet in shared memory
   l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 1);
   l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 2);
   l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 1);
   l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 2);
   float *sl = reinterpret_cast<float *>(smem + kVerifyStages * 2u * VT::kHalf + 16u * MT * VT::kPStride * 2u);   // the maxima's place
+  float *sref = sl + TS * 16u * MT;                                  // [16 MT]
   __syncthreads();
   if (t == 0u) {
     sl[th * 16u * MT + mt * 16u + g] = l_lo;
     sl[th * 16u * MT + mt * 16u + g + 8u] = l_hi;
+    if (th == 0u) {
+      sref[mt * 16u + g] = verify_rescale(ref_lo, m_lo) * (FP8 ? 1.f / kVerifyPScale : 1.f);
+      sref[mt * 16u + g + 8u] = verify_rescale(ref_hi, m_hi) * (FP8 ? 1.f / kVerifyPScale : 1.f);
+    }
   }
   __syncthreads();
   auto slot = [&](uint32_t row) {
@@ -768,6 +806,9 @@ attention_verify_kernel(const Params p) {
       if (row < m_rows) {
         float *dst = p.pacc + slot(row) * kD + 32u * warp + 8u * t;
         const int c = 2 * half;
+        const float last = sref[16u * a + g + 8u * half];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { o[a][j][c] *= last; o[a][j][c + 1] *= last; }
         if (p.vector_partials) {
           reinterpret_cast<float4 *>(dst)[0] = make_float4(o[a][0][c], o[a][1][c], o[a][2][c], o[a][3][c]);
           reinterpret_cast<float4 *>(dst)[1] = make_float4(o[a][0][c + 1], o[a][1][c + 1], o[a][2][c + 1], o[a][3][c + 1]);
@@ -892,9 +933,9 @@ int launch_verify_mt(const Params &p, uint32_t chunks) {
 // Rows of one kv head (tokens x q heads per kv head) decide the CTA's shape: one or two 16-row tiles; more, four per CTA
 // and as many CTAs (blockIdx.y) as that takes.  us a layer, split kernel + reduce, 24 / 4 heads, graph replay over cold
 // caches, with shared-memory expansion and ldmatrix operands before | now:
-//   FP8   5 tokens, context 1024 14.0 | 9.4   32768 47.7 | 26.7   131072 143.7 | 76.9   16 tokens, 32768 105.5 | 67.0
-//   BF16  5 tokens, context 1024 14.5 | 8.6   32768 40.0 | 31.3   131072 111.4 | 96.4   16 tokens, 32768  86.6 | 75.8
-// (bytes of 131072 rows at 6.65 TB/s: 40 us FP8, 81 us BF16; the rest of the FP8 time is the three barriers and the
+//   FP8   5 tokens, context 1024 14.0 | 8.3   32768 47.7 | 25.4   131072 143.7 |  78.0   16 tokens, 32768 105.5 | 67.7
+//   BF16  5 tokens, context 1024 14.5 | 7.2   32768 40.0 | 31.9   131072 111.4 | 102.7   16 tokens, 32768  86.6 | 75.8
+// (bytes of 131072 rows at 6.55 TB/s: 41 us FP8, 82 us BF16; the rest of the FP8 time is the three barriers and the
 // serial phases of a tile: eight warps, no overlap of one tile's scores with the P V of the one before).
 template <bool FP8>
 int launch_verify(const Params &p) {
