@@ -14,10 +14,11 @@
 // every other shape takes a general kernel (a CTA per q head and split).  One merge kernel (a CTA
 // per q head, launched with programmatic stream serialisation) combines the partials, adds the
 // current token in float32, writes the bf16 output and appends the row to the cache.  Without
-// partial buffers one CTA per q head walks the whole context and finishes the head itself.  The
+// partial buffers one CTA per q head walks the whole context, in float32 throughout, and finishes the head itself.  The
 // position may live on the device (position_device_i32), so no grid depends on it: a captured
-// graph stays valid while the context grows.  TurboQuant3 / 3.5 caches are not part of this
-// library.
+// graph stays valid while the context grows.  With partial buffers and the position on the host, a context that
+// fits the shared memory of one cluster per kv head takes one launch (below).  TurboQuant3 / 3.5 caches are not part
+// of this library.
 #include "common.cuh"
 
 #include <atomic>
@@ -1203,13 +1204,12 @@ extern "C" int qwen36_attention_decode(const qwen36_attention_decode_spec_t *spe
   a.head_dim = static_cast<uint32_t>(sh.head_dim);
   const bool fp8 = spec->kv_cache_dtype == kKvFp8;
   const bool partials = a.part_o != nullptr && a.part_m != nullptr && a.part_l != nullptr;
-  int one_status = QWEN36_STATUS_SUCCESS;
   if (partials && spec->decode_n_splits >= 2) {
     if (spec->split_timesteps_per_block != 0 && spec->split_timesteps_per_block < 64)
       return QWEN36_STATUS_INVALID_ARGUMENT;                       // attention.cu:2752-2754
+    int one_status = QWEN36_STATUS_SUCCESS;
     if (fp8 ? try_one_launch<true>(a, one_status) : try_one_launch<false>(a, one_status)) return one_status;
     return fp8 ? run_split_path<true>(a, spec->decode_n_splits) : run_split_path<false>(a, spec->decode_n_splits);
   }
-  if (fp8 ? try_one_launch<true>(a, one_status) : try_one_launch<false>(a, one_status)) return one_status;
   return fp8 ? launch_direct<true>(a) : launch_direct<false>(a);
 }

@@ -232,3 +232,24 @@ def test_one_launch_form_at_its_largest_contexts(backend, dtype, last):
     case = make_case(last + dtype, last + 1, 12, 2, 256, dtype)
     for position in (last // 2, last - 300, last - 16, last):
         run_and_check(backend, case, dtype, position, 64)
+
+
+def bf16_share_differing(backend, case, dtype, position):
+    q, k_new, v_new, ck, cv = case
+    got = backend.attention_decode(to_dev(q), to_dev(k_new), to_dev(v_new), cache_to_dev(ck), cache_to_dev(cv), position, dtype)
+    want = orc.attention_decode(q, k_new, v_new, ck.copy(), cv.copy(), dtype, position)
+    return float((bf16_host(got) != want).mean())
+
+
+@pytest.mark.parametrize("dtype", [BF16, FP8])
+@pytest.mark.parametrize("position", [63, 300, 1500])
+def test_without_partial_buffers_all_is_float32(backend, dtype, position):
+    """Scores, probabilities and sums in float32 leave the output within about 2e-6 of the oracle's, so one output in some
+    thousand falls on the other side of a bf16 rounding boundary (2^-8 apart); weights rounded to bf16 move a tenth of them, to
+    float16 one or two in a hundred.  0.5 %."""
+    assert bf16_share_differing(backend, make_case(position, position + 1, 24, 4, 256, dtype, q_gain=0.1), dtype, position) <= 0.005
+
+
+def test_without_partial_buffers_large_queries_over_fp8(backend):
+    """Queries past the largest float16: their scores are finite float32 numbers."""
+    run_and_check(backend, make_case(7, 301, 24, 4, 256, FP8, q_gain=2.0 ** 17), FP8, 300)
