@@ -694,18 +694,21 @@ decode_split_bf16_mma_kernel(const __nv_bfloat16 *__restrict__ q, const __nv_bfl
 // barriers, a second launch that fetches the partials back).  Here a cluster of CTAs owns a kv head; a CTA's whole share
 // of K and V is requested at once, so one memory latency covers it, and nothing is kept per warp that has to be merged:
 //   scores   a warp takes 16-token groups (the fragment plan of the split kernels); scores meet in shared memory
-//   softmax  a warp per q head: maximum, probabilities in the MMA operand order, sum
+//   softmax  a warp per q head: maximum, sum, and in the scores' place the probabilities as two 16-bit terms (the rounded
+//            value and what the rounding left), so that nothing is lost against the split kernels, whose warps each round
+//            against a maximum, and so an exact weight, of their own
 //   P V      a warp takes 32 dims over all of the CTA's tokens
 // The partial (m, l) pairs and output slices go straight from registers into the shared memory of the CTA that owns those
 // dims, one cluster barrier later every CTA finishes 256 / cluster dims of every head, the current token added in float32,
-// and appends them to the cache.  Operand formats are those of the split kernels (float16 q and probabilities for FP8,
-// bfloat16 for BF16), float32 everywhere else.  Sixteen warps: with eight, scores and P V took long enough to show from
-// 2000 tokens up (FP8 4097: 9.0 us, now 8.5).  Measured figures are at one_launch_cluster.
+// and appends them to the cache.  Operand formats are those of the split kernels (float16 for FP8, bfloat16 for BF16),
+// float32 everywhere else.  Sixteen warps: with eight, scores and P V took long enough to show from 2000 tokens up
+// (FP8 4097: 9.0 us against 8.5).  The second terms cost 2 - 3 % (FP8 4097: 8.7 -> 8.9, BF16 600: 5.0 -> 5.1).  Measured
+// figures are at one_launch_cluster.
 template <bool FP8> struct OneLaunch {
   static constexpr uint32_t kRowBytes = FP8 ? 256 : 512;
   static constexpr uint32_t kFixedBytes = 16 * 32 * 8 + 2 * 8 * 256 * 4 + 16 * 8 * 8 + 8 * 4;   // q fragments, slices, (m, l), scores of the new token
-  // K and V rows, eight float scores and eight 16-bit probabilities per token, with the row paddings of the latter two
-  static constexpr size_t smem_bytes(size_t tokens) { return tokens * (2 * kRowBytes + 48) + 8 * 8 * 4 + 8 * 8 * 2 + kFixedBytes; }
+  // K and V rows and eight float scores per token, with the row padding of the latter
+  static constexpr size_t smem_bytes(size_t tokens) { return tokens * (2 * kRowBytes + 32) + 8 * 8 * 4 + kFixedBytes; }
 };
 constexpr size_t kOneLaunchSmemLimit = 227 * 1024;
 constexpr int kOneThreads = 512, kOneWarps = kOneThreads / 32;
@@ -722,7 +725,7 @@ decode_one_launch_kernel(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat1
                          const __nv_bfloat16 *__restrict__ v_new, void *cache_k, void *cache_v,
                          __nv_bfloat16 *__restrict__ out, size_t position, uint32_t kv_heads, uint32_t tokens_per_cta) {
   constexpr uint32_t D = 256, RB = OneLaunch<FP8>::kRowBytes, CH = RB / 16;
-  constexpr float kPScale = FP8 ? 64.0f : 1.0f;
+  constexpr float kPScale = FP8 ? 32768.0f : 1.0f;                // float16 holds 65504
   const float sm_scale = 0.0625f * 1.4426950408889634f;           // rsqrt(256) * log2(e)
   extern __shared__ __align__(128) uint8_t smem[];
   const uint32_t T = tokens_per_cta;                              // a multiple of 16
@@ -731,9 +734,8 @@ decode_one_launch_kernel(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat1
   float *s_slices = reinterpret_cast<float *>(s_q + 16);          // [source CTA][half of its tokens][head][dims of this CTA]
   float2 (*s_ml)[8] = reinterpret_cast<float2 (*)[8]>(s_slices + 2 * 8 * 256);   // [source CTA][head]
   float *s_new = reinterpret_cast<float *>(s_ml + 16);            // scores of the current token, log2 units
-  const uint32_t SS = T + 8, PS = T + 8;                          // row strides of scores (float) and probabilities (16 bits)
+  const uint32_t SS = T + 8;                                      // row stride of the scores
   float *s_s = s_new + 8;
-  uint16_t *s_p = reinterpret_cast<uint16_t *>(s_s + 8 * SS);
 
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   const uint32_t g = lane >> 2, t = lane & 3u, slice = warp & 7u;
@@ -841,7 +843,7 @@ decode_one_launch_kernel(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat1
     __syncthreads();
     // ---- softmax of head `warp` over the CTA's tokens
     if (warp < G) {
-      const float2 *row = reinterpret_cast<const float2 *>(s_s + warp * SS);
+      float2 *row = reinterpret_cast<float2 *>(s_s + warp * SS);
       float mx = -INFINITY;
       for (uint32_t i = lane; i < groups * 8; i += 32) mx = fmaxf(mx, fmaxf(row[i].x, row[i].y));
       for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
@@ -850,14 +852,18 @@ decode_one_launch_kernel(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat1
         const float2 sc = row[i];
         const float p0 = sc.x == -INFINITY ? 0.f : exp2f(sc.x - mx), p1 = sc.y == -INFINITY ? 0.f : exp2f(sc.y - mx);
         sum += p0 + p1;
-        uint32_t packed;
+        uint2 terms;
         if (FP8) {
-          const __half2 h = __floats2half2_rn(p0 * kPScale, p1 * kPScale);
-          packed = *reinterpret_cast<const uint32_t *>(&h);
+          const float a = p0 * kPScale, b = p1 * kPScale;
+          const __half2 first = __floats2half2_rn(a, b);
+          const float2 f = __half22float2(first);
+          const __half2 rest = __floats2half2_rn(a - f.x, b - f.y);
+          terms = make_uint2(*reinterpret_cast<const uint32_t *>(&first), *reinterpret_cast<const uint32_t *>(&rest));
         } else {
-          packed = pack_bf16x2(p0, p1);
+          terms.x = pack_bf16x2(p0, p1);
+          terms.y = pack_bf16x2(p0 - __uint_as_float(terms.x << 16), p1 - __uint_as_float(terms.x & 0xffff0000u));
         }
-        *reinterpret_cast<uint32_t *>(s_p + warp * PS + 2 * i) = packed;
+        *reinterpret_cast<uint2 *>(row + i) = terms;
       }
       for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
       m = mx;
@@ -867,13 +873,11 @@ decode_one_launch_kernel(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat1
     __syncthreads();
     // ---- O^T = V^T P^T, dims 32 slice + 4 g + 2 j (row g), + 1 (row g + 8); warps 0 .. 7 take the even 16-token
     // groups, 8 .. 15 the odd ones
-#pragma unroll
-    for (int a = 0; a < 16; ++a) o[a >> 3][(a >> 2) & 1][a & 3] = 0.f;
-    auto multiply = [&](uint32_t grp, float (&acc)[2][4]) {
-      uint32_t b0 = 0u, b1 = 0u;
+    auto multiply = [&](uint32_t grp, float (&acc)[2][4], float (&rest)[2][4], bool two_terms) {
+      uint2 b0 = make_uint2(0u, 0u), b1 = b0;
       if (g < G) {
-        b0 = *reinterpret_cast<const uint32_t *>(s_p + g * PS + grp * 16 + 2 * t);
-        b1 = *reinterpret_cast<const uint32_t *>(s_p + g * PS + grp * 16 + 8 + 2 * t);
+        b0 = *reinterpret_cast<const uint2 *>(s_s + g * SS + grp * 16 + 2 * t);
+        b1 = *reinterpret_cast<const uint2 *>(s_s + g * SS + grp * 16 + 8 + 2 * t);
       }
       const uint8_t *vt = s_v + (grp * 16 + 2 * t) * RB;
       if (FP8) {
@@ -885,29 +889,45 @@ decode_one_launch_kernel(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat1
         e4m3x4_to_h2x2(__byte_perm(va, vb, 0x7362), ab2, ab3);
         e4m3x4_to_h2x2(__byte_perm(vc, vd, 0x5140), cd0, cd1);
         e4m3x4_to_h2x2(__byte_perm(vc, vd, 0x7362), cd2, cd3);
-        mma_f16(acc[0], ab0, ab1, cd0, cd1, b0, b1);
-        mma_f16(acc[1], ab2, ab3, cd2, cd3, b0, b1);
+        mma_f16(acc[0], ab0, ab1, cd0, cd1, b0.x, b1.x);
+        mma_f16(acc[1], ab2, ab3, cd2, cd3, b0.x, b1.x);
+        mma_f16(rest[0], ab0, ab1, cd0, cd1, b0.y, b1.y);
+        mma_f16(rest[1], ab2, ab3, cd2, cd3, b0.y, b1.y);
       } else {
         const uint32_t at = ((4 * slice + (g >> 1)) ^ (t << 1)) * 16 + (g & 1u) * 8;
         const uint2 va = *reinterpret_cast<const uint2 *>(vt + at), vb = *reinterpret_cast<const uint2 *>(vt + RB + at);
         const uint2 vc = *reinterpret_cast<const uint2 *>(vt + 8 * RB + at), vd = *reinterpret_cast<const uint2 *>(vt + 9 * RB + at);
-        mma_bf16(acc[0], __byte_perm(va.x, vb.x, 0x5410), __byte_perm(va.x, vb.x, 0x7632), __byte_perm(vc.x, vd.x, 0x5410),
-                 __byte_perm(vc.x, vd.x, 0x7632), b0, b1);
-        mma_bf16(acc[1], __byte_perm(va.y, vb.y, 0x5410), __byte_perm(va.y, vb.y, 0x7632), __byte_perm(vc.y, vd.y, 0x5410),
-                 __byte_perm(vc.y, vd.y, 0x7632), b0, b1);
+        const uint32_t ab0 = __byte_perm(va.x, vb.x, 0x5410), ab1 = __byte_perm(va.x, vb.x, 0x7632);
+        const uint32_t ab2 = __byte_perm(va.y, vb.y, 0x5410), ab3 = __byte_perm(va.y, vb.y, 0x7632);
+        const uint32_t cd0 = __byte_perm(vc.x, vd.x, 0x5410), cd1 = __byte_perm(vc.x, vd.x, 0x7632);
+        const uint32_t cd2 = __byte_perm(vc.y, vd.y, 0x5410), cd3 = __byte_perm(vc.y, vd.y, 0x7632);
+        mma_bf16(acc[0], ab0, ab1, cd0, cd1, b0.x, b1.x);
+        mma_bf16(acc[1], ab2, ab3, cd2, cd3, b0.x, b1.x);
+        if (two_terms) {
+          mma_bf16(rest[0], ab0, ab1, cd0, cd1, b0.y, b1.y);
+          mma_bf16(rest[1], ab2, ab3, cd2, cd3, b0.y, b1.y);
+        }
       }
     };
-    for (uint32_t grp = warp >> 3; grp < groups; grp += 4) {
-      multiply(grp, o[0]);
-      if (grp + 2 < groups) multiply(grp + 2, o[1]);
-    }
+    float probe;
+    for (bool two_terms = true;; two_terms = false) {
 #pragma unroll
-    for (int a = 0; a < 8; ++a) o[0][a >> 2][a & 3] += o[1][a >> 2][a & 3];
+      for (int a = 0; a < 16; ++a) o[a >> 3][(a >> 2) & 1][a & 3] = 0.f;
+      for (uint32_t grp = warp >> 3; grp < groups; grp += 4) {
+        multiply(grp, o[0], o[1], two_terms);
+        if (grp + 2 < groups) multiply(grp + 2, o[1], o[0], two_terms);
+      }
+      probe = 0.f;
+#pragma unroll
+      for (int a = 0; a < 8; ++a) {
+        o[0][a >> 2][a & 3] += o[1][a >> 2][a & 3];
+        probe += o[0][a >> 2][a & 3];
+      }
+      // BF16: a second term is zero or negative where the row may see an infinite V, so a NaN is looked at again without it
+      if (FP8 || !two_terms || !__any_sync(0xffffffffu, probe != probe)) break;
+    }
     if (!FP8 || pass == 1) break;
     // a NaN in the result: read the bytes 0x7F / 0xFF (which the append never writes) as +-448 and do it again
-    float probe = 0.f;
-#pragma unroll
-    for (int a = 0; a < 8; ++a) probe += o[0][a >> 2][a & 3];
     if (!__syncthreads_or(probe != probe)) break;
     for (uint32_t i = threadIdx.x; i < groups * 16 * CH; i += kOneThreads) {
       uint4 *k4 = reinterpret_cast<uint4 *>(s_k) + i, *v4 = reinterpret_cast<uint4 *>(s_v) + i;

@@ -253,3 +253,35 @@ def test_without_partial_buffers_all_is_float32(backend, dtype, position):
 def test_without_partial_buffers_large_queries_over_fp8(backend):
     """Queries past the largest float16: their scores are finite float32 numbers."""
     run_and_check(backend, make_case(7, 301, 24, 4, 256, FP8, q_gain=2.0 ** 17), FP8, 300)
+
+
+@pytest.mark.parametrize("position", [300, 1500])
+def test_bf16_cache_with_an_infinite_value(backend, position):
+    """A row of V with infinities in two dims: those outputs are infinite, the others as they were, whichever form runs."""
+    q, k_new, v_new, ck, cv = make_case(position, position + 1, 24, 4, 256, BF16, q_gain=0.05)
+    cv[7, 1, 3], cv[9, 1, 200] = 0x7F80, 0xFF80
+    for n_splits in (0, 16):
+        parts = partial_buffers(24, n_splits, 256) if n_splits else None
+        got = backend.attention_decode(to_dev(q), to_dev(k_new), to_dev(v_new), cache_to_dev(ck), cache_to_dev(cv), position, BF16,
+                                       parts, n_splits).float().cpu().numpy()
+        want = synth.bf16_bits_to_f32(orc.attention_decode(q, k_new, v_new, ck.copy(), cv.copy(), BF16, position))
+        assert np.isposinf(want[6:12, 3]).all() and np.isneginf(want[6:12, 200]).all()
+        finite = np.isfinite(want)
+        assert np.array_equal(got[~finite], want[~finite]) and rel_l2(got[finite], want[finite]) <= 1e-2
+
+
+@pytest.mark.parametrize("dtype", [BF16, FP8])
+@pytest.mark.parametrize("position", [600, 1500])
+def test_one_launch_form_loses_nothing_to_the_split_path(backend, dtype, position):
+    """Distance from the oracle (float32 throughout) on flat attention, where the rounding of the weights shows most: not
+    above the split path's, whose warps round against eight maxima."""
+    case = make_case(position + 3, position + 1, 24, 4, 256, dtype, q_gain=0.1)
+    q, k_new, v_new, ck, cv = case
+    err = []
+    try:
+        for mode in (1, 2):
+            backend.lib.qwen36_attention_decode_set_mode(mode)
+            err.append(run_and_check(backend, case, dtype, position, 64, tol=2.0 ** -8))
+    finally:
+        backend.lib.qwen36_attention_decode_set_mode(DEFAULT_MODE)
+    assert err[0] <= err[1]
