@@ -419,10 +419,14 @@ typedef struct {                         /* qwen36_fp4.h:108-147 */
  * are not read by this entry (nor by the reference's). */
 int qwen36_attention_flash_splitk_prefill_bf16(const qwen36_attention_prefill_spec_t *spec, int n_splits);
 /* Test hooks: mode 0 = general kernel only, 1 = tensor-core kernels where they
- * apply (default); n > 0 overrides the number of splits used. */
+ * apply (default), 2 = those without the one-launch form; n > 0 overrides the
+ * number of splits used.  _cluster reports what a call with this spec would do
+ * without doing it: the CTAs per kv head of the one-launch form, 0 for another
+ * form, -1 for a spec that is refused. */
 void qwen36_attention_decode_set_mode(int mode);
 void qwen36_attention_decode_force_splits(int n);
 void qwen36_attention_decode_force_cluster(int n);   /* 8 or 16: cluster size of the one-launch form, 0: by context */
+int qwen36_attention_decode_cluster(const qwen36_attention_decode_spec_t *spec);
 
 /* ---- additions of this build (no ABI change to anything above) ------------ */
 

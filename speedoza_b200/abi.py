@@ -309,6 +309,7 @@ def load() -> C.CDLL:
     lib.qwen36_attention_decode_force_splits.argtypes = [C.c_int]
     lib.qwen36_attention_decode_force_cluster.restype = None
     lib.qwen36_attention_decode_force_cluster.argtypes = [C.c_int]
+    lib.qwen36_attention_decode_cluster.argtypes = [C.POINTER(AttentionDecodeSpec)]
     lib.qwen36_nvfp4_chunk_gemv_set_mtile.restype = None
     lib.qwen36_nvfp4_matvec_force_quads.restype = None
     lib.qwen36_nvfp4_gemm_force_bn.restype = None

@@ -1071,27 +1071,28 @@ uint32_t pick_splits(const Args &a, size_t caller_splits, size_t ctas_per_split,
   return static_cast<uint32_t>(n);
 }
 
-// How many sixteen-CTA clusters the device can hold at once with all of the shared memory (0: none); asked once per device,
-// together with the permission for that cluster size.
+// How many clusters of `ctas` CTAs the device can hold at once with all of the shared memory (0: none); asked once per
+// device and size, together with the permission for sixteen.
 template <int G, bool FP8>
-int one_launch_clusters16() {
+uint32_t one_launch_clusters(uint32_t ctas) {
   static std::mutex mu;
-  static int known[64];                                           // count + 1; 0: not asked yet
+  static int known[64][2];                                        // count + 1; 0: not asked yet
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
   std::lock_guard<std::mutex> lock(mu);
-  if (known[dev] == 0) {
+  int &count = known[dev][ctas == 16];
+  if (count == 0) {
     int n = 0;
     const void *kernel = reinterpret_cast<const void *>(decode_one_launch_kernel<G, FP8>);
     if (q36::ensure_dynamic_smem(kernel, static_cast<int>(kOneLaunchSmemLimit)) == cudaSuccess &&
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+        (ctas <= 8 || cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)) {
       cudaLaunchConfig_t cfg{};
-      cfg.gridDim = dim3(16, 4);
+      cfg.gridDim = dim3(ctas, 4);
       cfg.blockDim = dim3(kOneThreads);
       cfg.dynamicSmemBytes = kOneLaunchSmemLimit;
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = 16;
+      attr[0].val.clusterDim.x = ctas;
       attr[0].val.clusterDim.y = 1;
       attr[0].val.clusterDim.z = 1;
       cfg.attrs = attr;
@@ -1101,26 +1102,32 @@ int one_launch_clusters16() {
         n = 0;
       }
     }
-    known[dev] = n + 1;
+    count = n + 1;
   }
-  return known[dev] - 1;
+  return static_cast<uint32_t>(count - 1);
 }
 
 // One launch or split + merge?  Returns the cluster size of the one-launch form, 0 for the split path.  The form needs the
-// context on the host (its shared memory is sized by it) and all of it in one cluster's shared memory; it was the faster
-// one wherever it fits.  us per layer, graph replay, 24 / 4 heads, split + merge | cluster of 8 | of 16:
-//   FP8   64 rows 7.2 | 4.5 | 4.7    400  9.5 | 4.9 | 5.0   1000  9.5 | 5.6 | 5.4   3000 10.3 |  -  | 7.3   5000 11.0 | - | 9.1
-//   BF16  64 rows 6.9 | 4.1 | 4.3    400 11.2 | 4.7 | 4.8   1000 11.6 | 5.6 | 5.3   2000 11.8 |  -  | 6.9   3000 12.0 | - | 8.1
-// (-: does not fit; eight CTAs hold half the rows).  Between the cluster sizes the line lies at 512 rows.
+// context on the host (its shared memory is sized by it), all of it in one cluster's shared memory, and a cluster per kv
+// head on the device at the same time: there it is the faster one throughout, in two rounds it is not.  us per layer,
+// graph replay, split + merge | cluster of 8 | of 16 (-: does not fit; eight CTAs hold half the rows):
+//   24 / 4 heads, FP8    64 rows 7.2 | 4.6 | 4.8    400  9.5 | 5.0 | 5.1   1000  9.5 | 5.8 | 5.5   3000 10.4 | 9.6 |  7.7   5000 11.1 |  -  |  9.5
+//                 BF16   64 rows 6.9 | 4.2 | 4.4    400 10.9 | 4.9 | 4.9   1000 11.6 | 6.0 | 5.5   2000 11.8 |  -  |  7.4   3000 12.1 |  -  |  8.7
+//   32 / 8 heads, FP8    64 rows 6.7 | 4.5 | 8.7    400  9.0 | 5.0 | 9.4   1000  9.0 | 5.8 | 10.1  3000 10.9 | 10.0 | 14.8  5000 13.7 |  -  | 18.3
+//   64 / 16 heads, FP8   64 rows 6.7 | 8.3 | 13.0   400  9.0 | 9.1 | 14.0  1000 10.4 | 12.6 | 17.7
+// (a B200 holds six or seven clusters of sixteen, twelve to fifteen of eight)
+// Between the cluster sizes the line lies at 512 rows.
 template <int G, bool FP8>
 uint32_t one_launch_cluster(const Args &a) {
   if (g_decode_mode != 1 || g_decode_force_splits > 0 || a.position_device != nullptr) return 0;
-  const int forced = g_one_launch_cluster.load();
-  uint32_t ctas = forced > 0 ? static_cast<uint32_t>(forced) : a.position > kOneLaunchWideFrom ? 16u : 8u;
-  const size_t per = q36::round_up(q36::div_ceil(a.position, ctas), 16);
-  if (OneLaunch<FP8>::smem_bytes(per < 16 ? 16 : per) > kOneLaunchSmemLimit) return 0;
-  if (ctas == 16 && one_launch_clusters16<G, FP8>() == 0) return 0;
-  return ctas;
+  auto fits = [&](uint32_t ctas) {
+    const size_t share = q36::round_up(q36::div_ceil(a.position, ctas), 16);
+    return OneLaunch<FP8>::smem_bytes(share < 16 ? 16 : share) <= kOneLaunchSmemLimit;
+  };
+  if (const uint32_t forced = static_cast<uint32_t>(g_one_launch_cluster.load()); forced != 0)
+    return fits(forced) && one_launch_clusters<G, FP8>(forced) != 0 ? forced : 0;
+  if (a.position > kOneLaunchWideFrom && fits(16) && a.kv_heads <= one_launch_clusters<G, FP8>(16)) return 16;
+  return fits(8) && a.kv_heads <= one_launch_clusters<G, FP8>(8) ? 8 : 0;
 }
 
 template <int G, bool FP8>
@@ -1147,16 +1154,17 @@ int launch_one(const Args &a, uint32_t ctas) {
                                              a.out, a.position, a.kv_heads, static_cast<uint32_t>(per)));
 }
 
+// The form's cluster size for this call (0: another form), and the launch.
 template <bool FP8>
-bool try_one_launch(const Args &a, int &status) {
+uint32_t try_one_launch(const Args &a, bool launch, int &status) {
   const bool aligned16 = ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.cache_k) |
                            reinterpret_cast<uintptr_t>(a.cache_v)) & 15u) == 0;
-  if (a.head_dim != 256 || !aligned16) return false;
+  if (a.head_dim != 256 || !aligned16) return 0;
 #define Q36_ONE(G) \
-  case G: { const uint32_t ctas = one_launch_cluster<G, FP8>(a); if (ctas == 0) return false; status = launch_one<G, FP8>(a, ctas); return true; }
+  case G: { const uint32_t ctas = one_launch_cluster<G, FP8>(a); if (ctas != 0 && launch) status = launch_one<G, FP8>(a, ctas); return ctas; }
   switch (a.q_per_kv) {
     Q36_ONE(1) Q36_ONE(2) Q36_ONE(4) Q36_ONE(6) Q36_ONE(8)
-    default: return false;
+    default: return 0;
   }
 #undef Q36_ONE
 }
@@ -1196,7 +1204,10 @@ extern "C" void qwen36_attention_decode_set_mode(int mode) { g_decode_mode = mod
 extern "C" void qwen36_attention_decode_force_cluster(int n) { g_one_launch_cluster = n == 8 || n == 16 ? n : 0; }
 extern "C" void qwen36_attention_decode_force_splits(int n) { g_decode_force_splits = n < 0 ? 0 : n; }
 
-extern "C" int qwen36_attention_decode(const qwen36_attention_decode_spec_t *spec) {
+namespace {
+
+// Checks the spec and runs it, or (cluster != nullptr) only reports the cluster size of the one-launch form, 0 for others.
+int decode(const qwen36_attention_decode_spec_t *spec, uint32_t *cluster) {
   if (spec == nullptr) return QWEN36_STATUS_NULL_POINTER;
   const qwen36_attention_shape_t &sh = spec->shape;
   // the reference's checks (kernels-cuda/attention.cu:2720-2734)
@@ -1228,8 +1239,23 @@ extern "C" int qwen36_attention_decode(const qwen36_attention_decode_spec_t *spe
     if (spec->split_timesteps_per_block != 0 && spec->split_timesteps_per_block < 64)
       return QWEN36_STATUS_INVALID_ARGUMENT;                       // attention.cu:2752-2754
     int one_status = QWEN36_STATUS_SUCCESS;
-    if (fp8 ? try_one_launch<true>(a, one_status) : try_one_launch<false>(a, one_status)) return one_status;
+    const bool launch = cluster == nullptr;
+    const uint32_t ctas = fp8 ? try_one_launch<true>(a, launch, one_status) : try_one_launch<false>(a, launch, one_status);
+    if (!launch) *cluster = ctas;
+    if (!launch || ctas != 0) return one_status;
     return fp8 ? run_split_path<true>(a, spec->decode_n_splits) : run_split_path<false>(a, spec->decode_n_splits);
   }
+  if (cluster != nullptr) { *cluster = 0; return QWEN36_STATUS_SUCCESS; }
   return fp8 ? launch_direct<true>(a) : launch_direct<false>(a);
+}
+
+}  // namespace
+
+extern "C" int qwen36_attention_decode(const qwen36_attention_decode_spec_t *spec) { return decode(spec, nullptr); }
+
+// Test hook: CTAs per kv head of the one-launch form if this call takes it, 0 if it takes another form, -1 for a spec that
+// is refused.
+extern "C" int qwen36_attention_decode_cluster(const qwen36_attention_decode_spec_t *spec) {
+  uint32_t ctas = 0;
+  return decode(spec, &ctas) == QWEN36_STATUS_SUCCESS ? static_cast<int>(ctas) : -1;
 }

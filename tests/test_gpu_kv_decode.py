@@ -1,12 +1,14 @@
 """GPU parity of qwen36_attention_decode (BF16 / FP8 E4M3 KV cache): output rel-L2 <= 1e-2
 against the oracle's restatement of the reference's float32 online softmax, cache append
 byte-exact (the appended row and nothing else changes)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
 
 from oracle import oracle as orc
-from speedoza_b200 import synth
+from speedoza_b200 import abi, synth
 from conftest import bf16_host, to_dev
 
 pytestmark = pytest.mark.gpu
@@ -172,7 +174,6 @@ def test_chained_steps_grow_the_cache(backend, dtype):
     ck_d, cv_d = cache_to_dev(ck), cache_to_dev(cv)
     pos_d = torch.tensor([start], dtype=torch.int32, device="cuda")
     parts = partial_buffers(q_heads, 16, head_dim)
-    from speedoza_b200 import abi
     for step in range(steps):
         q, k, v = synth.qkv(rng, 1, q_heads, kv_heads, head_dim)
         out = backend.attention_decode(to_dev(q), to_dev(k[0]), to_dev(v[0]), ck_d, cv_d, 0, dtype, parts, 16, pos_d)
@@ -206,7 +207,7 @@ def test_argument_checks(backend):
 @pytest.mark.parametrize("dtype", [BF16, FP8])
 @pytest.mark.parametrize("cluster", [8, 16])
 @pytest.mark.parametrize("position,q_heads,kv_heads", [
-    (0, 24, 4), (1, 24, 4), (15, 24, 4), (16, 8, 1), (127, 24, 4), (129, 24, 4), (300, 8, 8), (511, 8, 4), (1537, 24, 4)])
+    (0, 24, 4), (1, 24, 4), (15, 24, 4), (16, 8, 1), (127, 24, 4), (129, 24, 4), (300, 8, 8), (511, 8, 4), (1534, 24, 4)])
 def test_one_launch_form_equals_oracle_and_split_path(backend, dtype, cluster, position, q_heads, kv_heads):
     """Shares that are empty, ragged or whole, with both cluster sizes; the split path sees the same inputs.  Both round q
     (FP8) and the probabilities to 16 bits, so they differ by float32 orders and one rounding per probability; bf16 outputs: 2^-8."""
@@ -217,6 +218,7 @@ def test_one_launch_form_equals_oracle_and_split_path(backend, dtype, cluster, p
         for mode in (1, 2):
             backend.lib.qwen36_attention_decode_set_mode(mode)
             backend.lib.qwen36_attention_decode_force_cluster(cluster)
+            assert form(backend, dtype, position, q_heads, kv_heads) == (cluster if mode == 1 else 0)
             run_and_check(backend, case, dtype, position, 16)
             out.append(backend.attention_decode(to_dev(q), to_dev(k_new), to_dev(v_new), cache_to_dev(ck), cache_to_dev(cv),
                                                 position, dtype, partial_buffers(q_heads, 16, 256), 16).float())
@@ -226,12 +228,43 @@ def test_one_launch_form_equals_oracle_and_split_path(backend, dtype, cluster, p
         backend.lib.qwen36_attention_decode_force_cluster(0)
 
 
-@pytest.mark.parametrize("dtype,last", [(BF16, 3328), (FP8, 6528)])
-def test_one_launch_form_at_its_largest_contexts(backend, dtype, last):
-    """Around the context where the shared memory of a cluster ends and the split path takes over."""
-    case = make_case(last + dtype, last + 1, 12, 2, 256, dtype)
-    for position in (last // 2, last - 300, last - 16, last):
+def form(backend, dtype, position, q_heads=24, kv_heads=4, splits=64, block=0):
+    """CTAs per kv head of the one-launch form if a call of these sizes takes it, 0 if it takes another form."""
+    a = torch.zeros(64, device="cuda").data_ptr()
+    spec = abi.AttentionDecodeSpec(0, position, *(abi.DevicePtr(a) for _ in range(5)), abi.DevicePtr(0), abi.DevicePtr(a),
+                                   abi.AttentionShape(q_heads, kv_heads, 256, 0), dtype, abi.DevicePtr(0),
+                                   *(abi.DevicePtr(a) for _ in range(3)), splits, block)
+    return backend.lib.qwen36_attention_decode_cluster(C.byref(spec))
+
+
+@pytest.mark.parametrize("dtype,tokens", [(BF16, 192), (FP8, 384)])
+def test_one_launch_form_at_its_largest_contexts(backend, dtype, tokens):
+    """Up to, at and past the context where the shared memory of a cluster ends (`tokens` cached rows per CTA: K, V and
+    eight float scores each in what 227 KB leave beside 21.8 KB) and the split path takes over."""
+    assert tokens == (227 * 1024 - 21536 - 256) // (32 + (512 if dtype == FP8 else 1024)) // 16 * 16
+    last = 16 * tokens
+    case = make_case(last + dtype, last + 2, 12, 2, 256, dtype)
+    for position, ctas in ((last - 300, 16), (last - 1, 16), (last, 16), (last + 1, 0)):
+        assert form(backend, dtype, position, 12, 2) == ctas
         run_and_check(backend, case, dtype, position, 64)
+    last = 8 * tokens
+    try:
+        backend.lib.qwen36_attention_decode_force_cluster(8)
+        for position, ctas in ((last - 1, 8), (last, 8), (last + 1, 0)):
+            assert form(backend, dtype, position, 12, 2) == ctas
+            run_and_check(backend, case, dtype, position, 64)
+    finally:
+        backend.lib.qwen36_attention_decode_force_cluster(0)
+
+
+@pytest.mark.parametrize("dtype", [BF16, FP8])
+@pytest.mark.parametrize("q_heads,kv_heads", [(24, 4), (32, 8), (64, 16), (32, 32)])
+def test_one_launch_form_only_where_every_kv_head_has_a_cluster_at_once(backend, dtype, q_heads, kv_heads):
+    """A B200 holds six or seven clusters of sixteen and twelve to fifteen of eight with all of their shared memory."""
+    assert form(backend, dtype, 300, q_heads, kv_heads) == (8 if kv_heads <= 8 else 0)
+    assert form(backend, dtype, 1500, q_heads, kv_heads) == (16 if kv_heads <= 4 else 8 if kv_heads <= 8 else 0)
+    for position in (300, 1500):
+        run_and_check(backend, make_case(q_heads + dtype, position + 1, q_heads, kv_heads, 256, dtype), dtype, position, 64)
 
 
 def bf16_share_differing(backend, case, dtype, position):
@@ -247,6 +280,7 @@ def test_without_partial_buffers_all_is_float32(backend, dtype, position):
     """Scores, probabilities and sums in float32 leave the output within about 2e-6 of the oracle's, so one output in some
     thousand falls on the other side of a bf16 rounding boundary (2^-8 apart); weights rounded to bf16 move a tenth of them, to
     float16 one or two in a hundred.  0.5 %."""
+    assert form(backend, dtype, position, splits=1) == 0
     assert bf16_share_differing(backend, make_case(position, position + 1, 24, 4, 256, dtype, q_gain=0.1), dtype, position) <= 0.005
 
 
@@ -281,6 +315,7 @@ def test_one_launch_form_loses_nothing_to_the_split_path(backend, dtype, positio
     try:
         for mode in (1, 2):
             backend.lib.qwen36_attention_decode_set_mode(mode)
+            assert form(backend, dtype, position) == (16 if mode == 1 else 0)
             err.append(run_and_check(backend, case, dtype, position, 64, tol=2.0 ** -8))
     finally:
         backend.lib.qwen36_attention_decode_set_mode(DEFAULT_MODE)
