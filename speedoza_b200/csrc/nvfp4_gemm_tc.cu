@@ -237,6 +237,23 @@ nvfp4_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_base_slot, 0);
   const uint32_t tmem_sf = tmem_base + C::kAccStages * C::kAccCols;
+
+  uint32_t pf_tile = blockIdx.x, pf_kb = 0;
+  auto prefetch_one = [&]() {
+    if (pf_tile >= tiles) return;
+    tma_prefetch_2d(&map_a, pf_kb * kBKBytes, (pf_tile / n_blocks) * kBM);
+    bulk_prefetch(a_sf + (static_cast<size_t>(pf_tile / n_blocks) * sf_tiles_per_block + pf_kb * 4u) * 512u, 2048u);
+    if (++pf_kb == k_blocks) { pf_kb = 0; pf_tile += gridDim.x; }
+  };
+  // Launched while the kernel ahead drains: nothing may be read before that kernel is done (a caller may have
+  // produced either operand just now), but asking L2 for the weights of the first stages reads nothing.  Five
+  // tokens, graph replay over cold weights: gate_up 34816 x 5120 20.7 -> 18.9 us.
+  if (threadIdx.x == 0)
+    for (uint32_t i = 0; i < kAhead + C::kStages; ++i) prefetch_one();
+  // Every role waits, so that no bounded wait below counts the time of the kernel ahead, and the trigger comes behind the
+  // wait: a GEMV launched next streams its weights before its own wait, and would otherwise do so while the kernel
+  // ahead of THIS one is still writing them.
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (warp == 0) {
@@ -244,19 +261,6 @@ nvfp4_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     if (lane == 0) {
       uint32_t g = 0;
       bool dead = false;
-      uint32_t pf_tile = blockIdx.x, pf_kb = 0;
-      auto prefetch_one = [&]() {
-        if (pf_tile >= tiles) return;
-        tma_prefetch_2d(&map_a, pf_kb * kBKBytes, (pf_tile / n_blocks) * kBM);
-        bulk_prefetch(a_sf + (static_cast<size_t>(pf_tile / n_blocks) * sf_tiles_per_block + pf_kb * 4u) * 512u, 2048u);
-        if (++pf_kb == k_blocks) { pf_kb = 0; pf_tile += gridDim.x; }
-      };
-      for (uint32_t i = 0; i < kAhead; ++i) prefetch_one();
-      // Launched while the kernel ahead drains: nothing may be read before that kernel is done (a caller may have
-      // produced either operand just now), but asking L2 for the weights of the first stages reads nothing.  Five
-      // tokens, graph replay over cold weights: gate_up 34816 x 5120 20.7 -> 18.9 us.
-      for (uint32_t i = 0; i < C::kStages; ++i) prefetch_one();
-      asm volatile("griddepcontrol.wait;" ::: "memory");
       for (uint32_t tile = blockIdx.x; tile < tiles && !dead; tile += gridDim.x) {
         const uint32_t nb = tile % n_blocks, mb = tile / n_blocks;
         for (uint32_t kb = 0; kb < k_blocks; ++kb, ++g) {
@@ -361,7 +365,6 @@ nvfp4_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     const uint32_t col0 = ((warp - kWarpEpilogue) >> 2) * C::kEpiCols;   // first accumulator column of this warp
     uint32_t t_local = 0;
     bool dead = false;
-    asm volatile("griddepcontrol.wait;" ::: "memory");    // the output may still be in use by the kernel ahead
     for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++t_local) {
       const uint32_t nb = tile % n_blocks, mb = tile / n_blocks;
       const uint32_t as = t_local % C::kAccStages, aph = (t_local / C::kAccStages) & 1u;
@@ -1162,17 +1165,19 @@ nvfp4_gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 #pragma unroll
   for (uint32_t j = 0; j < kCols; ++j) acc[j] = 0.f;
   bool ok = true;
+  // as in the persistent kernel: L2 is asked for the first weights while the kernel ahead drains (down 5120 x 17408 at
+  // five tokens: 13.9 -> 13.4 us), every role waits, and the trigger comes behind the wait
+  if (threadIdx.x == 0) {
+    for (uint32_t kb = kb_begin; kb < kb_end && kb < kb_begin + C::kStages + 2u; ++kb) {
+      tma_prefetch_2d(&map_a, kb * kBKBytes, mb * kBM);
+      bulk_prefetch(a_sf + (static_cast<size_t>(mb) * sf_tiles_per_block + kb * 4u) * 512u, 2048u);
+    }
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (warp == 0) {
     if (lane == 0) {
-      // as in the persistent kernel: L2 is asked for the first weights while the kernel ahead drains (down
-      // 5120 x 17408 at five tokens: 13.9 -> 13.4 us)
-      for (uint32_t kb = kb_begin; kb < kb_end && kb < kb_begin + C::kStages + 2u; ++kb) {
-        tma_prefetch_2d(&map_a, kb * kBKBytes, mb * kBM);
-        bulk_prefetch(a_sf + (static_cast<size_t>(mb) * sf_tiles_per_block + kb * 4u) * 512u, 2048u);
-      }
-      asm volatile("griddepcontrol.wait;" ::: "memory");
       for (uint32_t kb = kb_begin, g = 0; kb < kb_end; ++kb, ++g) {
         const uint32_t s = g % C::kStages, ph = (g / C::kStages) & 1u;
         if (!mbar_wait(&empty[s], ph ^ 1u)) break;
@@ -1228,7 +1233,6 @@ nvfp4_gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   } else if (warp >= kWarpEpilogue && warp < kWarpEpilogue + 4u) {
     // epilogue warps 4..7: drain this CTA's partial sums; ranks > 0 hand them to the first CTA
     const uint32_t quarter = warp & 3u;
-    asm volatile("griddepcontrol.wait;" ::: "memory");    // the output may still be in use by the kernel ahead
     if (kb_end > kb_begin) {
       ok = mbar_wait(&acc_full[0], 0u);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

@@ -1,0 +1,33 @@
+"""Launch order of the kernels that start while the kernel ahead drains, read from the sources.
+
+The GEMVs stream their weights before they wait for the kernel ahead, so a weight must be complete by the time
+the kernel ahead of the GEMV lets it in.  A kernel that lets its dependents in only behind its own wait vouches
+for everything before itself; one that does so earlier lets them reach further back."""
+import glob
+import os
+import re
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+TRIGGER, WAIT = "griddepcontrol.launch_dependents", "griddepcontrol.wait"
+
+# Let their dependents in ahead of their own wait.  The two GEMVs do it from the producer warp.  The two reductions only
+# ever follow their own split kernel, which lets them in behind ITS wait and writes nothing but their partials.
+EARLY = {"nvfp4_gemv_mma_kernel", "nvfp4_matvec_kernel", "attention_splitk_reduce_kernel", "attention_few_splits_reduce_kernel"}
+
+
+def kernels():
+    """name -> body of every __global__ function under csrc (bodies end at a closing brace in the first column)."""
+    found = {}
+    for path in sorted(glob.glob(os.path.join(ROOT, "speedoza_b200", "csrc", "*.cu"))):
+        text = re.sub(r"//[^\n]*", "", open(path).read())
+        for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\([^\n]*\)\s+)?(\w+)\s*\(", text):
+            found[m.group(1)] = text[m.end():text.index("\n}", m.end())]
+    return found
+
+
+def test_dependents_are_let_in_behind_the_wait():
+    bodies = kernels()
+    assert {"nvfp4_gemm_tc_kernel", "nvfp4_gemm_splitk_kernel", "nvfp4_gemm_pair6_kernel"} <= set(bodies) and EARLY <= set(bodies)
+    early = {name for name, body in bodies.items()
+             if TRIGGER in body and WAIT in body and body.index(TRIGGER) < body.index(WAIT)}
+    assert early == EARLY
