@@ -74,6 +74,12 @@ inline int sm_count_current_device() {
 __host__ __device__ static inline size_t div_ceil(size_t a, size_t b) { return (a + b - 1) / b; }
 __host__ __device__ static inline size_t round_up(size_t a, size_t b) { return div_ceil(a, b) * b; }
 
+// The kernels that quantise rows write what may be a weight, and the GEMVs read their weights before they wait for the
+// kernel ahead.  So they let the next kernel in before they are complete only with fewer rows than this, and a GEMV over a
+// matrix of fewer rows starts when the kernel ahead is complete.  (Whole scale tiles; every form but the plain matvec takes
+// multiples of 128 rows.  Five activation rows: with the trigger a feed-forward block takes 1.7 us less.)
+constexpr uint32_t kWeightRows = 128;
+
 // Tiled block-scale layout (kernels-cuda/ops.cu:64-79): 128 outer rows x 4
 // inner groups form one 512-byte tile; inside it row r sits at
 // (r % 32) * 16 + (r / 32) * 4 and the 4 groups are adjacent bytes.  Tiles of

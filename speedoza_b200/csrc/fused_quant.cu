@@ -376,7 +376,7 @@ swiglu_nvfp4_quantize_rows_kernel(const __nv_bfloat16 *__restrict__ gate, const 
   const uint32_t group = blockIdx.x * 32u + (threadIdx.x >> 1), half = threadIdx.x & 1u;
   const bool in_row = group < groups;
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (rows < q36::kWeightRows) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0 && tensor_scale != nullptr) *tensor_scale = g;
 
   const uint32_t row_step = gridDim.y * 4u;

@@ -446,7 +446,7 @@ int launch_kernel(const qwen36_nvfp4_matvec_spec_t *s, const CUtensorMap &map_w,
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = N < q36::kWeightRows ? 0 : 1;
   return q36::cuda_status(cudaLaunchKernelEx(
       &cfg, nvfp4_matvec_kernel<QUADS, TMAP>, map_w, map_sf, as_ptr<const __nv_bfloat16>(s->input_bf16),
       as_ptr<const uint8_t>(s->weight_u8), as_ptr<const uint8_t>(s->block_scale_e4m3),

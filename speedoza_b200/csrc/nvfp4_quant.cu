@@ -29,7 +29,7 @@ nvfp4_quantize_kernel(const __nv_bfloat16 *__restrict__ in, uint8_t *__restrict_
                       uint8_t *__restrict__ out_sf, float *__restrict__ tensor_scale, Index rows,
                       Index values, float input_tensor_scale) {
   asm volatile("griddepcontrol.wait;" ::: "memory");               // launched with programmatic stream serialisation
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (rows < q36::kWeightRows) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const float g = input_tensor_scale > 0.0f ? input_tensor_scale : 1.0f;
   const Index groups = (values + 15) / 16;
   const Index padded = (groups + 3) / 4 * 4;
@@ -157,7 +157,7 @@ nvfp4_quantize_fast_kernel(const __nv_bfloat16 *__restrict__ in, uint8_t *__rest
   const uint32_t group = blockIdx.x * 64u + threadIdx.x;
   const bool in_row = group < groups;
   asm volatile("griddepcontrol.wait;" ::: "memory");               // launched with programmatic stream serialisation
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (rows < q36::kWeightRows) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0 && tensor_scale != nullptr) *tensor_scale = g;
 
   // A thread walks several rows; the two 16-byte loads of the next row are issued before the current

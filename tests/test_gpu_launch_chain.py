@@ -18,12 +18,12 @@ def rows(gen, *shape):
     return torch.randn(shape, generator=gen, device="cuda").to(torch.bfloat16)
 
 
-@pytest.mark.parametrize("m,k", [(1024, 5120), (34816, 5120)])
-@pytest.mark.parametrize("tokens", [5, 100])
+@pytest.mark.parametrize("m,k", [(64, 5120), (1024, 5120), (34816, 5120)])
+@pytest.mark.parametrize("tokens", [0, 5, 100])
 def test_weight_quantised_ahead_of_its_gemv(backend, m, k, tokens):
     """A matrix is quantised on the device and multiplied by the one-token kernel, which streams its weights before it
-    waits for the kernel ahead, with a product of other weights in between (split-K form at 5 tokens, one CTA per tile
-    at 100)."""
+    waits for the kernel ahead: directly behind the quantiser, and with a product of other weights in between (split-K form at
+    5 tokens, one CTA per tile at 100)."""
     gen = torch.Generator(device="cuda").manual_seed(m + tokens)
     ws = [rows(gen, m, k) for _ in range(3)]
     x, acts = rows(gen, k), rows(gen, max(tokens, 1), k)

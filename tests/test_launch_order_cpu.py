@@ -31,3 +31,13 @@ def test_dependents_are_let_in_behind_the_wait():
     early = {name for name, body in bodies.items()
              if TRIGGER in body and WAIT in body and body.index(TRIGGER) < body.index(WAIT)}
     assert early == EARLY
+
+
+def test_writers_of_weight_format_are_complete_first():
+    """Row quantisers let the next kernel in early only for fewer rows than a GEMV that starts early takes."""
+    bodies = kernels()
+    for name in ("nvfp4_quantize_kernel", "nvfp4_quantize_fast_kernel", "swiglu_nvfp4_quantize_rows_kernel"):
+        lines = [line.strip() for line in bodies[name].splitlines() if TRIGGER in line]
+        assert all(line.startswith("if (rows < q36::kWeightRows)") for line in lines), name
+    launch = open(os.path.join(ROOT, "speedoza_b200", "csrc", "nvfp4_matvec.cu")).read()
+    assert "cfg.numAttrs = N < q36::kWeightRows ? 0 : 1;" in launch
