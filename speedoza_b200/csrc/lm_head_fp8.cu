@@ -917,6 +917,7 @@ argmax_rows_kernel(const __nv_bfloat16 *__restrict__ logits, uint32_t *__restric
   __shared__ float c_val[kArgmaxCluster];
   __shared__ uint32_t c_idx[kArgmaxCluster];
 
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // "this CTA runs": waited for before the remote stores
   const size_t row = blockIdx.x / kArgmaxCluster;
   const uint32_t rank = cluster.block_rank();
   const __nv_bfloat16 *l = logits + row * vocab;
@@ -948,6 +949,8 @@ argmax_rows_kernel(const __nv_bfloat16 *__restrict__ logits, uint32_t *__restric
     }
   }
   for (size_t i = head + vec * 8 + tid; i < vocab; i += nthreads) consider(__bfloat162float(l[i]), static_cast<uint32_t>(i));
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
 
   for (int off = 16; off > 0; off >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, bv, off);

@@ -161,6 +161,7 @@ top8_rescore_kernel(const WsEntry *__restrict__ ws, const __nv_bfloat16 *__restr
   if (staged) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
   const size_t row = staged ? blockIdx.x / kCandidates : blockIdx.x;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  if (staged) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // "this CTA runs": waited for before the remote stores
   asm volatile("griddepcontrol.wait;" ::: "memory");               // launched with programmatic stream serialisation
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
@@ -170,6 +171,8 @@ top8_rescore_kernel(const WsEntry *__restrict__ ws, const __nv_bfloat16 *__restr
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(rows_smem + c * 2))),
                    "l"(x_row + c) : "memory");
     asm volatile("cp.async.commit_group;" ::: "memory");
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
   }
   float max_v2 = -INFINITY;
   for (uint32_t b = threadIdx.x; b < kBlocks; b += kThreads) {

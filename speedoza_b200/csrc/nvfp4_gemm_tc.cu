@@ -1137,6 +1137,7 @@ nvfp4_gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   float *partials = reinterpret_cast<float *>(stages + C::kStages * C::kStageBytes);   // [S-1][128 rows][kCols], first CTA only
 
   const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31u;
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // "this CTA runs": waited for before the remote stores
   uint32_t S, rank;
   asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(S));
   S = __shfl_sync(0xffffffffu, S, 0);
@@ -1173,6 +1174,8 @@ nvfp4_gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       bulk_prefetch(a_sf + (static_cast<size_t>(mb) * sf_tiles_per_block + kb * 4u) * 512u, 2048u);
     }
   }
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 

@@ -1,4 +1,4 @@
-"""Launch order of the kernels that start while the kernel ahead drains, read from the sources.
+"""Order of waits in the kernels, read from the sources: those that start while the kernel ahead drains, and clusters.
 
 The GEMVs stream their weights before they wait for the kernel ahead, so a weight must be complete by the time
 the kernel ahead of the GEMV lets it in.  A kernel that lets its dependents in only behind its own wait vouches
@@ -41,3 +41,15 @@ def test_writers_of_weight_format_are_complete_first():
         assert all(line.startswith("if (rows < q36::kWeightRows)") for line in lines), name
     launch = open(os.path.join(ROOT, "speedoza_b200", "csrc", "nvfp4_matvec.cu")).read()
     assert "cfg.numAttrs = N < q36::kWeightRows ? 0 : 1;" in launch
+
+
+def test_remote_shared_memory_only_once_the_cluster_runs():
+    """Stores into another CTA's shared memory come behind a cluster barrier: all CTAs of the cluster have started."""
+    remote = re.compile(r"map_to_cta\(|cluster_rank_address\(|mapa\.shared|map_shared_rank\(")
+    barrier = re.compile(r"cluster_sync_all\(|barrier\.cluster\.wait")
+    found = {}
+    for name, body in kernels().items():
+        if remote.search(body):
+            first = barrier.search(body)
+            found[name] = first is not None and first.start() < remote.search(body).start()
+    assert len(found) >= 6 and all(found.values()), found
