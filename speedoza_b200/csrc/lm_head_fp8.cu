@@ -1055,7 +1055,7 @@ bool bound_route(size_t rows, size_t cols, size_t n, size_t workspace_bytes, siz
 template <int N, bool FUSED>
 int launch_gemv_n(const uint8_t *w, const float *scales, const __nv_bfloat16 *x, __nv_bfloat16 *y, size_t rows,
                   size_t cols, uint32_t row_offset, uint32_t *tokens, float *best, float2 *partials,
-                  unsigned *ticket, unsigned grid) {
+                  unsigned *ticket, unsigned grid, size_t slots) {
   if constexpr (N >= 2 && N <= 8) {
     if (stage_f32(N, cols)) {
       // (2..8 tokens gain 7-40 % on the float16 route, fused or not: two tokens 352 -> 260 us; one token is
@@ -1068,7 +1068,8 @@ int launch_gemv_n(const uint8_t *w, const float *scales, const __nv_bfloat16 *x,
         if (q36::ensure_dynamic_smem(reinterpret_cast<const void *>(lm_head_gemv_f16_kernel<N, FUSED>), 200 * 1024) != cudaSuccess)
           return QWEN36_STATUS_CUDA_ERROR;
         const size_t need = q36::div_ceil(rows, static_cast<size_t>(kWarps) * kF16Rows);
-        const size_t cap = static_cast<size_t>(sm_count()) * 2;
+        size_t cap = static_cast<size_t>(sm_count()) * 2;
+        if (FUSED && cap > slots) cap = slots;                     // every CTA leaves its winners in the caller's workspace
         lm_head_gemv_f16_kernel<N, FUSED><<<static_cast<unsigned>(need < cap ? need : cap), kThreads, smem16, q36::stream()>>>(
             w, scales, x, y, rows, static_cast<uint32_t>(cols), row_offset, tokens, best, partials, ticket);
         if (q36::launch_status() != QWEN36_STATUS_SUCCESS) return QWEN36_STATUS_CUDA_ERROR;
@@ -1085,20 +1086,6 @@ int launch_gemv_n(const uint8_t *w, const float *scales, const __nv_bfloat16 *x,
   return launch_gemv_x<N, FUSED, false>(w, scales, x, y, rows, cols, row_offset, tokens, best, partials, ticket, grid);
 }
 
-template <bool FUSED>
-int launch_gemv(size_t n, const uint8_t *w, const float *scales, const __nv_bfloat16 *x, __nv_bfloat16 *y,
-                size_t rows, size_t cols, uint32_t row_offset, uint32_t *tokens, float *best, float2 *partials,
-                unsigned *ticket, unsigned grid) {
-#define Q36_CASE(NN) \
-  case NN: return launch_gemv_n<NN, FUSED>(w, scales, x, y, rows, cols, row_offset, tokens, best, partials, ticket, grid);
-  switch (n) {
-    Q36_CASE(1) Q36_CASE(2) Q36_CASE(3) Q36_CASE(4) Q36_CASE(5) Q36_CASE(6) Q36_CASE(7) Q36_CASE(8)
-    Q36_CASE(9) Q36_CASE(10) Q36_CASE(11) Q36_CASE(12) Q36_CASE(13) Q36_CASE(14) Q36_CASE(15) Q36_CASE(16)
-    default: return QWEN36_STATUS_INVALID_ARGUMENT;
-  }
-#undef Q36_CASE
-}
-
 // Persistent grid: enough CTAs to fill the GPU, never more than there is work.
 unsigned gemv_grid(size_t rows, size_t n, size_t cols) {
   const bool f32 = stage_f32(n, cols);
@@ -1108,6 +1095,22 @@ unsigned gemv_grid(size_t rows, size_t n, size_t cols) {
   const size_t per_sm = smem > 100 * 1024 ? 1 : (smem > 48 * 1024 ? 2 : 4);
   const size_t cap = static_cast<size_t>(sm_count()) * per_sm;
   return static_cast<unsigned>(need < cap ? need : cap);
+}
+
+template <bool FUSED>
+int launch_gemv(size_t n, const uint8_t *w, const float *scales, const __nv_bfloat16 *x, __nv_bfloat16 *y,
+                size_t rows, size_t cols, uint32_t row_offset, uint32_t *tokens, float *best, float2 *partials,
+                unsigned *ticket, size_t slots) {
+  unsigned grid = gemv_grid(rows, n, cols);
+  if (FUSED && grid > slots) grid = static_cast<unsigned>(slots);
+#define Q36_CASE(NN) \
+  case NN: return launch_gemv_n<NN, FUSED>(w, scales, x, y, rows, cols, row_offset, tokens, best, partials, ticket, grid, slots);
+  switch (n) {
+    Q36_CASE(1) Q36_CASE(2) Q36_CASE(3) Q36_CASE(4) Q36_CASE(5) Q36_CASE(6) Q36_CASE(7) Q36_CASE(8)
+    Q36_CASE(9) Q36_CASE(10) Q36_CASE(11) Q36_CASE(12) Q36_CASE(13) Q36_CASE(14) Q36_CASE(15) Q36_CASE(16)
+    default: return QWEN36_STATUS_INVALID_ARGUMENT;
+  }
+#undef Q36_CASE
 }
 
 bool gemv_args_ok(size_t rows, size_t cols, size_t n, uint64_t w, uint64_t s, uint64_t x) {
@@ -1143,7 +1146,7 @@ extern "C" int qwen36_lm_head_fp8_gemv(const qwen36_lm_head_fp8_gemv_spec_t *spe
     const int rc = launch_gemv<false>(nt, as_ptr<const uint8_t>(spec->weight_e4m3), as_ptr<const float>(spec->row_scales_f32),
                                       as_ptr<const __nv_bfloat16>(spec->input_bf16) + t0 * spec->cols,
                                       as_ptr<__nv_bfloat16>(spec->output_bf16) + t0 * spec->rows, spec->rows, spec->cols, 0u,
-                                      nullptr, nullptr, nullptr, nullptr, gemv_grid(spec->rows, nt, spec->cols));
+                                      nullptr, nullptr, nullptr, nullptr, 0);
     if (rc != QWEN36_STATUS_SUCCESS) return rc;
   }
   return QWEN36_STATUS_SUCCESS;
@@ -1166,8 +1169,6 @@ extern "C" int qwen36_lm_head_fp8_gemv_argmax(const qwen36_lm_head_fp8_argmax_sp
   // the ticket (it is back at zero when a launch ends) and the winners' slots
   for (size_t t0 = 0; t0 < spec->n; t0 += kChunkTokens) {
     const size_t nt = spec->n - t0 < kChunkTokens ? spec->n - t0 : kChunkTokens;
-    unsigned grid = gemv_grid(spec->rows, nt, spec->cols);
-    if (grid > slots) grid = static_cast<unsigned>(slots);
     float *best = as_ptr<float>(spec->best_value_f32);
     if (bound_route(spec->rows, spec->cols, nt, spec->workspace_bytes, spec->n)) {
       int rc = QWEN36_STATUS_INVALID_ARGUMENT;
@@ -1192,7 +1193,7 @@ extern "C" int qwen36_lm_head_fp8_gemv_argmax(const qwen36_lm_head_fp8_argmax_sp
                                      spec->cols, spec->row_offset, as_ptr<uint32_t>(spec->output_token_u32) + t0,
                                      best == nullptr ? nullptr : best + t0,
                                      reinterpret_cast<float2 *>(static_cast<uintptr_t>(spec->workspace.ptr + 16)),
-                                     as_ptr<unsigned>(spec->workspace), grid);
+                                     as_ptr<unsigned>(spec->workspace), slots);
     if (rc != QWEN36_STATUS_SUCCESS) return rc;
   }
   return QWEN36_STATUS_SUCCESS;

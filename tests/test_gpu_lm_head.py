@@ -181,3 +181,17 @@ def test_bound_and_refine_picks_the_exact_winner(backend, n, cols, kind):
         tok, best = backend.lm_head_fp8_gemv_argmax(wd, sd, xd, scratch, row_offset=77)
         assert np.array_equal(tok.cpu().numpy().astype(np.uint32), want + 77)
         assert np.array_equal(best.cpu().numpy(), np.where(np.isnan(best_want), -np.inf, best_want))
+
+
+@pytest.mark.parametrize("n", [1, 2, 4, 8, 9])
+def test_fused_argmax_stays_inside_a_small_workspace(backend, n):
+    """A workspace with room for the winners of five CTAs: as many run, and nothing behind it is written."""
+    rows, cols = 6563, 5120
+    rng = np.random.default_rng(n)
+    w, s = synth.lm_head_weight(rng, rows, cols)
+    x = synth.activations(rng, n, cols)
+    buf = torch.zeros(1 << 16, dtype=torch.uint8, device="cuda")
+    buf[16 + 5 * 8 * n:] = 0xA5
+    tok, _ = backend.lm_head_fp8_gemv_argmax(to_dev(w), to_dev(s), to_dev(x), buf[: 16 + 5 * 8 * n])
+    assert np.array_equal(tok.cpu().numpy().astype(np.uint32), orc.argmax_rows(orc.lm_head_fp8_gemv(w, s, x)))
+    assert bool((buf[16 + 5 * 8 * n:] == 0xA5).all())
