@@ -613,10 +613,12 @@ int qwen36_argmax_peer_combine(const qwen36_argmax_peer_combine_spec_t *spec);
  * best_value_f32 (optional) receives the winning bf16 logit as float per
  * token, for the cross-shard combine.  workspace: at least
  * qwen36_lm_head_fp8_argmax_workspace_bytes(rows, n) bytes, zero-filled once
- * before first use (the kernel leaves its counter zeroed; the rest is scratch).
- * With that much, calls of four or more tokens on a large weight bound every
- * row on the tensor cores and evaluate only the rows that can win; a smaller
- * workspace (16 + 8 n bytes per CTA used, at least one) keeps the exact scan. */
+ * before first use (a call leaves the first sixteen bytes zeroed; the rest is
+ * scratch).  With that much, calls of four or more tokens on a large weight
+ * bound every row on the tensor cores and evaluate only the rows that can win,
+ * with the exact scan behind them for inputs that bounds do not tell apart; a
+ * smaller workspace (16 bytes, and 8 n for each CTA used, at least one) keeps
+ * the exact scan. */
 typedef struct {
   size_t rows, cols, n;
   qwen36_device_ptr_t weight_e4m3, row_scales_f32, input_bf16;

@@ -215,6 +215,21 @@ __device__ __forceinline__ bool x_fits_f16(const __nv_bfloat16 *__restrict__ x, 
   return fit;
 }
 
+// An exact scan that stands behind a bound-and-refine launch (gate != nullptr): it is launched with programmatic stream
+// serialisation and does its work only where that launch asked for it.  The first of the launches clears the bound
+// kernel's counter for the next call.
+struct Gate {
+  const unsigned *redo;
+  unsigned *counter;
+};
+__device__ __forceinline__ bool gate_closed(const Gate gate) {
+  if (gate.redo == nullptr) return false;
+  if (gate.counter != nullptr) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the other scan, which waits first
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (gate.counter != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *gate.counter = 0u;
+  return __ldcg(gate.redo) == 0u;
+}
+
 // UNFIT_ONLY: the launch that follows a float16-route launch on the same inputs; it returns at
 // once when that one did the work.
 template <int N, bool FUSED, bool XF32, bool UNFIT_ONLY = false>
@@ -223,8 +238,9 @@ lm_head_gemv_kernel(const uint8_t *__restrict__ weight, const float *__restrict_
                     const __nv_bfloat16 *__restrict__ x, __nv_bfloat16 *__restrict__ y, size_t rows,
                     uint32_t cols, uint32_t row_offset, uint32_t *__restrict__ out_tokens,
                     float *__restrict__ out_best, float2 *__restrict__ partials,
-                    unsigned *__restrict__ ticket) {
+                    unsigned *__restrict__ ticket, const Gate gate) {
   constexpr int R = RowsPerWarp<N, XF32>::value;
+  if (FUSED && gate_closed(gate)) return;
   extern __shared__ __align__(16) uint8_t smem[];
   uint4 *xs = reinterpret_cast<uint4 *>(smem);        // N * cols bf16, swizzled chunks
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -366,8 +382,9 @@ lm_head_gemv_f16_kernel(const uint8_t *__restrict__ weight, const float *__restr
                         const __nv_bfloat16 *__restrict__ x, __nv_bfloat16 *__restrict__ y, size_t rows,
                         uint32_t cols, uint32_t row_offset, uint32_t *__restrict__ out_tokens,
                         float *__restrict__ out_best, float2 *__restrict__ partials,
-                        unsigned *__restrict__ ticket) {
+                        unsigned *__restrict__ ticket, const Gate gate) {
   constexpr int R = kF16Rows;
+  if (FUSED && gate_closed(gate)) return;
   constexpr int S = F16Ring<N>::kStages;
   extern __shared__ __align__(16) uint8_t smem[];
   uint4 *xs = reinterpret_cast<uint4 *>(smem);        // N * cols float16, swizzled 16-byte chunks
@@ -492,7 +509,7 @@ lm_head_gemv_f16_kernel(const uint8_t *__restrict__ weight, const float *__restr
 //
 // The reference's logit is a float32 FMA chain, which no tensor-core product reproduces bit for bit, and at a
 // few tokens that chain (one FMA per weight and token) costs more than the weight's bytes (four tokens, 248320 x
-// 5120: 342 us against 191 us of HBM time).  The argmax needs the exact chain only where a row can win:
+// 5120: 339 us against 194 us of HBM time).  The argmax needs the exact chain only where a row can win:
 //   1. lm_head_bound_kernel multiplies on the tensor cores (float16 operands, float32 accumulation: E4M3 ->
 //      float16 is exact, bf16 -> float16 times the token's power of two is exact for the values within 2^28 of
 //      the largest and off by at most 2^-25 for the rest).  Beside it runs a bound on A = sum |w x|: the sum of |w|
@@ -506,14 +523,21 @@ lm_head_gemv_f16_kernel(const uint8_t *__restrict__ weight, const float *__restr
 //   2. lm_head_refine_kernel: rounding to bf16 is monotone, so a row whose rounded hi lies below the largest
 //      rounded lo of the token cannot win and cannot tie.  The others (the winner and, with N(0,1) logits, a
 //      row or two) get the reference's chain; the winner among them is the winner among all rows, bit for bit.
-// An all-zero token's logits are exact zeros already (its rows all tie): its hi is its value.  With infinities, NaN or
-// magnitudes outside 2^-100 .. 2^100 among the activations the bound kernel evaluates the reference's chain for every
-// row instead, and hi is the value for all tokens.
+//   3. The exact scan, launched behind the two and gone at once unless they ask for it, because bounds do not help:
+//      - infinities, NaN or magnitudes outside 2^-100 .. 2^100 among the activations (nothing is bounded then);
+//      - flat logits (equal rows, a zeroed weight): every warp of the bound kernel looks whether the first sixteen rows it
+//        bounds can be told apart; when a quarter of the warps cannot, the others stop after the rows they are at;
+//      - more candidates than kMaxExact for one warp of the refine kernel (many near-copies of the best row).
+//      248320 x 5120, four tokens: with equal rows 445 us, 6000 near-copies of the best row in one place 605, an infinity 393,
+//      where the exact scan alone takes 339 (381 with the infinity) and the bounds, where they help, 270.
+// An all-zero token's logits are exact zeros already (its rows all tie): its hi is its value.
 constexpr int kBoundThreads = 768;
 constexpr int kBoundWarps = kBoundThreads / 32;
 constexpr uint32_t kBoundStageBytes = 16 * 128;                  // sixteen rows x 128 columns
 constexpr unsigned kBoundMaxCtas = 256;
 constexpr int kBoundStages = 3;
+constexpr int kMaxExact = 16;                                    // exact sums per warp of the refine kernel: about 2 us each
+constexpr unsigned kBadInput = 1u << 31;                         // beside the tokens' bits in the flags word
 constexpr size_t kBoundSmemLimit = 230720;                       // beside up to 1.7 KB of static shared memory
 constexpr size_t bound_smem_bytes(size_t n, size_t cols) {
   return n * cols * 2 + static_cast<size_t>(kBoundWarps) * kBoundStages * kBoundStageBytes + cols / 4;
@@ -524,6 +548,12 @@ __device__ __forceinline__ void bound_groups(size_t rows, uint32_t b, uint32_t c
   const uint64_t groups = (rows + 15) / 16;
   first = static_cast<uint32_t>(groups * b / ctas);
   last = static_cast<uint32_t>(groups * (b + 1) / ctas);
+}
+
+// Warps whose first sixteen rows must be indistinguishable for the exact scan to take over: a quarter of those with rows.
+__device__ __forceinline__ unsigned flat_limit(size_t rows, uint32_t ctas) {
+  const size_t groups = (rows + 15) / 16, warps = static_cast<size_t>(ctas) * kBoundWarps;
+  return static_cast<unsigned>((groups < warps ? groups : warps) / 4);
 }
 
 // The reference's logit of one (row, token), by a whole warp: the chain of lm_head_gemv_kernel.
@@ -557,12 +587,13 @@ __device__ __forceinline__ float exact_logit(const uint8_t *__restrict__ weight,
 // A warp owns a 16-row group at a time and a cp.async ring in which a lane reads back only what it copied itself;
 // the ring runs on across groups.  24 warps: with sixteen the latency of a stage's
 // dependent steps showed (285 against 270 us for the whole call).  It is issue slots that bound it now (3.5 per weight, half
-// of them busy), not bytes: 240 us of 191.  Figures at bound_route.
+// of them busy), not bytes: 240 us of 194.  Figures at bound_route.
 template <int N>
 __global__ void __launch_bounds__(kBoundThreads, 1)
 lm_head_bound_kernel(const uint8_t *__restrict__ weight, const float *__restrict__ row_scales,
                      const __nv_bfloat16 *__restrict__ x, size_t rows, uint32_t cols, float *__restrict__ hi_out,
-                     float2 *__restrict__ cta_bounds, float *__restrict__ warp_hi, unsigned *__restrict__ flags) {
+                     float2 *__restrict__ cta_bounds, float *__restrict__ warp_hi, unsigned *__restrict__ flags,
+                     unsigned *__restrict__ redo, unsigned *__restrict__ flat) {
   constexpr int S = kBoundStages;
   extern __shared__ __align__(16) uint8_t smem[];
   uint4 *xs = reinterpret_cast<uint4 *>(smem);     // [64-column block][half][t][token]: four columns of two MMA steps
@@ -637,34 +668,13 @@ lm_head_bound_kernel(const uint8_t *__restrict__ weight, const float *__restrict
   }
   __syncthreads();
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    unsigned f = 0u;
-    for (int k = 0; k < N; ++k) f |= s_bad || s_max[k] == 0u ? 1u << k : 0u;
+    unsigned f = s_bad ? kBadInput : 0u;
+    for (int k = 0; k < N; ++k) f |= s_max[k] == 0u ? 1u << k : 0u;
     *flags = f;
+    *redo = 0u;
   }
-  if (s_bad) {                                                    // every logit by the reference's chain, no bounds
+  if (s_bad) {                                                    // no bounds: the exact scan does the work
     q36::cp_async_wait<0>();
-    float top[N];
-#pragma unroll
-    for (int k = 0; k < N; ++k) top[k] = -INFINITY;
-    const size_t end = min(rows, static_cast<size_t>(grp_last) * 16);
-    for (uint32_t grp = grp_first + warp; grp < grp_last; grp += kBoundWarps)      // (the groups that are this warp's below)
-      for (size_t row = static_cast<size_t>(grp) * 16; row < min(end, static_cast<size_t>(grp) * 16 + 16); ++row) {
-#pragma unroll
-        for (int k = 0; k < N; ++k) {
-          const float v = exact_logit(weight, row_scales, x + static_cast<size_t>(k) * cols, row, cols);
-          if (lane == 0) hi_out[k * rows + row] = v;
-          top[k] = fmaxf(top[k], v);
-        }
-      }
-#pragma unroll
-    for (int k = 0; k < N; ++k)
-      if (lane == 0) { s_bound[warp][k] = make_float2(top[k], top[k]); warp_hi[(blockIdx.x * kBoundWarps + warp) * 8u + k] = top[k]; }
-    __syncthreads();
-    if (threadIdx.x < N) {
-      float t = s_bound[0][threadIdx.x].x;
-      for (int w = 1; w < kBoundWarps; ++w) t = fmaxf(t, s_bound[w][threadIdx.x].x);
-      cta_bounds[blockIdx.x * 8u + threadIdx.x] = make_float2(t, t);
-    }
     return;
   }
   {
@@ -700,7 +710,10 @@ lm_head_bound_kernel(const uint8_t *__restrict__ weight, const float *__restrict
   }
 
   uint32_t slot = 0;
-  for (uint32_t grp = 0; grp < mine; ++grp) {
+  const unsigned limit = flat_limit(rows, gridDim.x);
+  bool stop = false;
+  for (uint32_t grp = 0; grp < mine && !stop; ++grp) {
+    const unsigned seen = *reinterpret_cast<volatile unsigned *>(flat);      // looked at a few steps later
     const size_t row0 = (static_cast<size_t>(grp_first) + warp + grp * kBoundWarps) * 16 + g;
     float scale[2];
 #pragma unroll
@@ -709,6 +722,7 @@ lm_head_bound_kernel(const uint8_t *__restrict__ weight, const float *__restrict
 #pragma unroll
     for (int i = 0; i < 16; ++i) d[i >> 2][i & 3] = 0.f;
     for (uint32_t step = 0; step < steps; ++step) {
+      if (step == 4u && __shfl_sync(0xffffffffu, seen, 0) > limit) { stop = true; break; }
       q36::cp_async_wait<S - 2>();                                // this lane's own copies of the stage
       const uint32_t at = ring + slot * kBoundStageBytes;
       const uint4 w0[2] = {q36::lds128(at), q36::lds128(at + 512u)};               // row g, both 64-column blocks
@@ -742,11 +756,13 @@ lm_head_bound_kernel(const uint8_t *__restrict__ weight, const float *__restrict
         mag[1] = fmaf(su.x + su.y, xm, mag[1]);
       }
     }
+    if (stop) break;
 #pragma unroll
     for (int r = 0; r < 2; ++r) {                                 // the quad's lanes hold the row's columns between them
       mag[r] += __shfl_xor_sync(0xffffffffu, mag[r], 1);
       mag[r] += __shfl_xor_sync(0xffffffffu, mag[r], 2);
     }
+    float low[2][2], high[2][2];                                  // of the group's rows, for its first group: see `flat`
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       const size_t row = row0 + 8 * r;
@@ -764,14 +780,33 @@ lm_head_bound_kernel(const uint8_t *__restrict__ weight, const float *__restrict
           hi = base + margin;
           if (hi != hi && sum == sum && s == s) { lo = -INFINITY; hi = INFINITY; }
         }
-        if (k < N && row < rows) {
+        const bool counts = k < N && row < rows;
+        if (counts) {
           hi_out[k * rows + row] = hi;                            // NaN stays NaN: such a row cannot win
           best_lo[e] = fmaxf(best_lo[e], lo);
           best_hi[e] = fmaxf(best_hi[e], hi);
         }
+        low[r][e] = lo;
+        high[r][e] = counts && !zero[e] ? hi : NAN;
       }
     }
+    if (grp == 0) {
+      // rows that could still be the first sixteen's winner, after the rounding to bf16 that the refine kernel compares
+      uint32_t possible[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float top = fmaxf(low[0][e], low[1][e]);
+#pragma unroll
+        for (int off = 16; off >= 4; off >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
+        top = __bfloat162float(__float2bfloat16(top));
+        possible[e] = (__bfloat162float(__float2bfloat16(high[0][e])) >= top) + (__bfloat162float(__float2bfloat16(high[1][e])) >= top);
+#pragma unroll
+        for (int off = 16; off >= 4; off >>= 1) possible[e] += __shfl_xor_sync(0xffffffffu, possible[e], off);
+      }
+      if (__any_sync(0xffffffffu, possible[0] >= 12u || possible[1] >= 12u) && lane == 0) atomicAdd(flat, 1u);
+    }
   }
+  q36::cp_async_wait<0>();                                        // a warp that stopped early has copies in flight
 #pragma unroll
   for (int e = 0; e < 2; ++e) {
 #pragma unroll
@@ -801,14 +836,18 @@ __global__ void __launch_bounds__(kThreads, 1)
 lm_head_refine_kernel(const uint8_t *__restrict__ weight, const float *__restrict__ row_scales,
                       const __nv_bfloat16 *__restrict__ x, size_t rows, uint32_t cols, const float *__restrict__ hi,
                       const float2 *__restrict__ cta_bounds, const float *__restrict__ warp_hi,
-                      const unsigned *__restrict__ flags, uint32_t row_offset,
-                      uint32_t *__restrict__ out_tokens, float *__restrict__ out_best, float2 *__restrict__ partials,
-                      unsigned *__restrict__ ticket) {
+                      const unsigned *__restrict__ flags, unsigned *__restrict__ redo, const unsigned *__restrict__ flat,
+                      uint32_t row_offset, uint32_t *__restrict__ out_tokens, float *__restrict__ out_best,
+                      float2 *__restrict__ partials, unsigned *__restrict__ ticket) {
   __shared__ float s_lo[kWarps][N];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const unsigned flag = __ldcg(flags);
+  if ((flag & kBadInput) != 0u || __ldcg(flat) > flat_limit(rows, gridDim.x)) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *redo = 1u;
+    return;
+  }
   // thread b looks at CTA b's bounds: the largest lo of all decides which CTAs have rows to look at
   float lo[N], hi_max[N], need[N];
 #pragma unroll
@@ -840,14 +879,15 @@ lm_head_refine_kernel(const uint8_t *__restrict__ weight, const float *__restric
   for (int k = 0; k < N; ++k) { best[k] = -INFINITY; best_idx[k] = 0u; }
   uint32_t grp_first, grp_last;
   bound_groups(rows, blockIdx.x, gridDim.x, grp_first, grp_last);
-  for (uint32_t bw = warp; bw < static_cast<uint32_t>(kBoundWarps); bw += kWarps) {     // a warp of the bound kernel and its groups
+  int left = kMaxExact;                                           // below zero: too many, the exact scan does the work
+  for (uint32_t bw = warp; bw < static_cast<uint32_t>(kBoundWarps) && left >= 0; bw += kWarps) {     // a warp of the bound kernel and its groups
     bool any = false;
 #pragma unroll
     for (int k = 0; k < N; ++k)
       any |= __bfloat162float(__float2bfloat16(__ldcg(warp_hi + (blockIdx.x * kBoundWarps + bw) * 8u + k))) >= need[k];
     if (!any) continue;
     constexpr int kAhead = 4;                                     // pairs of groups whose hi values are requested together
-    for (uint32_t grp0 = grp_first + bw; grp0 < grp_last; grp0 += 2 * kAhead * kBoundWarps) {
+    for (uint32_t grp0 = grp_first + bw; grp0 < grp_last && left >= 0; grp0 += 2 * kAhead * kBoundWarps) {
       float h[kAhead][N];
       size_t row[kAhead];
 #pragma unroll
@@ -858,23 +898,30 @@ lm_head_refine_kernel(const uint8_t *__restrict__ weight, const float *__restric
 #pragma unroll
         for (int k = 0; k < N; ++k) h[p][k] = in ? __ldcg(hi + k * rows + row[p]) : NAN;
       }
+      uint32_t wanted[kAhead], pairs = 0u;                        // tokens whose exact logit a row needs; such pairs of this lane
 #pragma unroll
       for (int p = 0; p < kAhead; ++p) {
-        uint32_t wanted = 0u;                                     // tokens whose exact logit this row needs
+        wanted[p] = 0u;
 #pragma unroll
         for (int k = 0; k < N; ++k) {
           if ((flag >> k) & 1u) {                                 // hi is the logit
             const uint32_t idx = static_cast<uint32_t>(row[p]) + row_offset;
             if (better(h[p][k], idx, best[k], best_idx[k])) { best[k] = h[p][k]; best_idx[k] = idx; }
           } else if (__bfloat162float(__float2bfloat16(h[p][k])) >= need[k]) {
-            wanted |= 1u << k;
+            wanted[p] |= 1u << k;
           }
         }
-        uint32_t lanes = __ballot_sync(0xffffffffu, wanted != 0u);
+        pairs += __popc(wanted[p]);
+      }
+      left -= static_cast<int>(__reduce_add_sync(0xffffffffu, pairs));
+      if (left < 0) break;
+#pragma unroll
+      for (int p = 0; p < kAhead; ++p) {
+        uint32_t lanes = __ballot_sync(0xffffffffu, wanted[p] != 0u);
         while (lanes != 0u) {
           const int src = __ffs(lanes) - 1;
           lanes &= lanes - 1u;
-          const uint32_t todo = __shfl_sync(0xffffffffu, wanted, src);
+          const uint32_t todo = __shfl_sync(0xffffffffu, wanted[p], src);
           const uint32_t at = __shfl_sync(0xffffffffu, static_cast<uint32_t>(row[p]), src);     // below 2^32, as tokens are
 #pragma unroll
           for (int k = 0; k < N; ++k)
@@ -886,6 +933,7 @@ lm_head_refine_kernel(const uint8_t *__restrict__ weight, const float *__restric
       }
     }
   }
+  if (left < 0 && lane == 0) *redo = 1u;
 #pragma unroll
   for (int k = 0; k < N; ++k)
 #pragma unroll
@@ -999,34 +1047,42 @@ int sm_count() { return q36::sm_count_current_device(); }
 bool stage_f32(size_t n, size_t cols) { return n >= 2 && n <= 8 && n * cols * 4 <= 200 * 1024; }
 size_t stage_bytes(size_t n, size_t cols) { return n * cols * (stage_f32(n, cols) ? 4 : 2); }
 
+// A scan over the whole weight, or one that stands behind a bound-and-refine launch (see Gate).
+template <typename... KArgs, typename... Args>
+int launch_scan(void (*kernel)(KArgs...), size_t grid, size_t smem, const Gate &gate, Args... args) {
+  if (q36::ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), 200 * 1024) != cudaSuccess) return QWEN36_STATUS_CUDA_ERROR;
+  if (gate.redo != nullptr)
+    return q36::cuda_status(q36::launch_after_previous(kernel, dim3(static_cast<unsigned>(grid)), dim3(kThreads), smem, q36::stream(), args..., gate));
+  kernel<<<static_cast<unsigned>(grid), kThreads, smem, q36::stream()>>>(args..., gate);
+  return q36::launch_status();
+}
+
 template <int N, bool FUSED, bool XF32>
 int launch_gemv_x(const uint8_t *w, const float *scales, const __nv_bfloat16 *x, __nv_bfloat16 *y, size_t rows,
                   size_t cols, uint32_t row_offset, uint32_t *tokens, float *best, float2 *partials,
-                  unsigned *ticket, unsigned grid) {
-  const size_t smem = static_cast<size_t>(N) * cols * (XF32 ? 4 : 2);
-  if (q36::ensure_dynamic_smem(reinterpret_cast<const void *>(lm_head_gemv_kernel<N, FUSED, XF32>), 200 * 1024) != cudaSuccess)
-    return QWEN36_STATUS_CUDA_ERROR;
-  lm_head_gemv_kernel<N, FUSED, XF32><<<grid, kThreads, smem, q36::stream()>>>(
-      w, scales, x, y, rows, static_cast<uint32_t>(cols), row_offset, tokens, best, partials, ticket);
-  return q36::launch_status();
+                  unsigned *ticket, unsigned grid, const Gate &gate) {
+  return launch_scan(lm_head_gemv_kernel<N, FUSED, XF32>, grid, static_cast<size_t>(N) * cols * (XF32 ? 4 : 2), gate, w, scales, x, y,
+                     rows, static_cast<uint32_t>(cols), row_offset, tokens, best, partials, ticket);
 }
 
 std::atomic<int> g_gemv_route{0};      // test hook: 1 = float32 route only, 2 = no bound-and-refine
 
 constexpr size_t kBoundMinBytes = 32u << 20, kBoundMinTokens = 4;
 
-// Scratch of the bound-and-refine route behind the ticket and the CTA winners: flags word (bit k: token k's hi values are its logits), bounds of the
-// CTAs and of their warps, hi values.
+// Scratch of the bound-and-refine route behind the ticket and the CTA winners: flags word (bit k: token k's hi values are its
+// logits), redo word (the exact scan is to do the work), bounds of the CTAs and of their warps, hi values.
 constexpr size_t kChunkTokens = 8;      // tokens per launch: the float16 and bound-and-refine routes' limit
 size_t winners_bytes(size_t n) { return 16 + static_cast<size_t>(148 * 4) * 8 * (n == 0 ? 1 : n); }
 size_t bound_scratch_bytes(size_t rows, size_t n) {
   return 16 + kBoundMaxCtas * 8 * (sizeof(float2) + kBoundWarps * sizeof(float)) + (n < kChunkTokens ? n : kChunkTokens) * rows * sizeof(float);
 }
 
+// Words of the workspace that the route needs beside its scratch: the ticket and, zero between calls as well, the counter of
+// the bound kernel (both in the first sixteen bytes).
 template <int N>
 int launch_bound(const uint8_t *w, const float *scales, const __nv_bfloat16 *x, size_t rows, size_t cols,
                  uint32_t row_offset, uint32_t *tokens, float *best, float2 *partials, unsigned *ticket, uint8_t *scratch) {
-  unsigned *flags = reinterpret_cast<unsigned *>(scratch);
+  unsigned *flags = reinterpret_cast<unsigned *>(scratch), *redo = flags + 1, *flat = ticket + 1;
   float2 *bounds = reinterpret_cast<float2 *>(scratch + 16);
   float *warp_hi = reinterpret_cast<float *>(bounds + kBoundMaxCtas * 8), *hi = warp_hi + kBoundMaxCtas * 8 * kBoundWarps;
   const unsigned sms = static_cast<unsigned>(sm_count());
@@ -1034,18 +1090,19 @@ int launch_bound(const uint8_t *w, const float *scales, const __nv_bfloat16 *x, 
   if (q36::ensure_dynamic_smem(reinterpret_cast<const void *>(lm_head_bound_kernel<N>), static_cast<int>(kBoundSmemLimit)) != cudaSuccess)
     return QWEN36_STATUS_CUDA_ERROR;
   lm_head_bound_kernel<N><<<grid, kBoundThreads, bound_smem_bytes(N, cols), q36::stream()>>>(
-      w, scales, x, rows, static_cast<uint32_t>(cols), hi, bounds, warp_hi, flags);
+      w, scales, x, rows, static_cast<uint32_t>(cols), hi, bounds, warp_hi, flags, redo, flat);
   if (q36::launch_status() != QWEN36_STATUS_SUCCESS) return QWEN36_STATUS_CUDA_ERROR;
   return q36::cuda_status(q36::launch_after_previous(lm_head_refine_kernel<N>, dim3(grid), dim3(kThreads), 0, q36::stream(), w,
-                                                     scales, x, rows, static_cast<uint32_t>(cols), hi, bounds, warp_hi, flags, row_offset,
-                                                     tokens, best, partials, ticket));
+                                                     scales, x, rows, static_cast<uint32_t>(cols), hi, bounds, warp_hi, flags, redo, flat,
+                                                     row_offset, tokens, best, partials, ticket));
 }
 
 // Does the bound-and-refine route take this call?  It needs its scratch (callers that hold less keep the exact scan),
 // whole 128-column stages, and enough tokens and weight.  us, bounds + refine | exact scan:
-//   248320 x 5120: 3 tokens 299 | 281   4 tokens 266 | 358   6 tokens 270 | 464   8 tokens 311 | 624
-//   100000 x 4096: 4 tokens 102 | 128   60000 x 2048: 4 tokens 50 | 54, 8 tokens 61 | 89
-//   16384 x 2048 (32 MB): 4 tokens 23 | 29, 8 tokens 28 | 44
+//   248320 x 5120: 3 tokens 299 | 281   4 tokens 272 | 339   6 tokens 277 | 460   8 tokens 315 | 615
+//   100000 x 4096: 4 tokens 109 | 127   8 tokens 126 | 228   60000 x 2048: 4 tokens 54.5 | 53.3   8 tokens 64 | 87
+//   16384 x 2048 (32 MB): 4 tokens 25 | 28   8 tokens 33 | 42
+// Eight tokens end at 5120 columns, where the activations and the ring just fit shared memory: wider, the exact scan.
 bool bound_route(size_t rows, size_t cols, size_t n, size_t workspace_bytes, size_t n_call) {
   return g_gemv_route.load() == 0 && n >= kBoundMinTokens && cols % 128 == 0 && rows * cols >= kBoundMinBytes && rows < (1ull << 32) - 16 &&
          bound_smem_bytes(n, cols) <= kBoundSmemLimit &&
@@ -1055,7 +1112,7 @@ bool bound_route(size_t rows, size_t cols, size_t n, size_t workspace_bytes, siz
 template <int N, bool FUSED>
 int launch_gemv_n(const uint8_t *w, const float *scales, const __nv_bfloat16 *x, __nv_bfloat16 *y, size_t rows,
                   size_t cols, uint32_t row_offset, uint32_t *tokens, float *best, float2 *partials,
-                  unsigned *ticket, unsigned grid, size_t slots) {
+                  unsigned *ticket, unsigned grid, size_t slots, const Gate &gate) {
   if constexpr (N >= 2 && N <= 8) {
     if (stage_f32(N, cols)) {
       // (2..8 tokens gain 7-40 % on the float16 route, fused or not: two tokens 352 -> 260 us; one token is
@@ -1065,25 +1122,19 @@ int launch_gemv_n(const uint8_t *w, const float *scales, const __nv_bfloat16 *x,
         // float16 route first; the float32 route right behind it runs only for activations the
         // float16 route declines (both decide on the same data, on the device, so nothing is read back)
         const size_t smem16 = static_cast<size_t>(N) * cols * 2 + static_cast<size_t>(kWarps) * F16Ring<N>::kStages * kF16StageBytes;
-        if (q36::ensure_dynamic_smem(reinterpret_cast<const void *>(lm_head_gemv_f16_kernel<N, FUSED>), 200 * 1024) != cudaSuccess)
-          return QWEN36_STATUS_CUDA_ERROR;
         const size_t need = q36::div_ceil(rows, static_cast<size_t>(kWarps) * kF16Rows);
         size_t cap = static_cast<size_t>(sm_count()) * 2;
         if (FUSED && cap > slots) cap = slots;                     // every CTA leaves its winners in the caller's workspace
-        lm_head_gemv_f16_kernel<N, FUSED><<<static_cast<unsigned>(need < cap ? need : cap), kThreads, smem16, q36::stream()>>>(
-            w, scales, x, y, rows, static_cast<uint32_t>(cols), row_offset, tokens, best, partials, ticket);
-        if (q36::launch_status() != QWEN36_STATUS_SUCCESS) return QWEN36_STATUS_CUDA_ERROR;
-        const size_t smem = static_cast<size_t>(N) * cols * 4;
-        if (q36::ensure_dynamic_smem(reinterpret_cast<const void *>(lm_head_gemv_kernel<N, FUSED, true, true>), 200 * 1024) != cudaSuccess)
-          return QWEN36_STATUS_CUDA_ERROR;
-        lm_head_gemv_kernel<N, FUSED, true, true><<<grid, kThreads, smem, q36::stream()>>>(
-            w, scales, x, y, rows, static_cast<uint32_t>(cols), row_offset, tokens, best, partials, ticket);
-        return q36::launch_status();
+        const int rc = launch_scan(lm_head_gemv_f16_kernel<N, FUSED>, need < cap ? need : cap, smem16, gate, w, scales, x, y, rows,
+                                   static_cast<uint32_t>(cols), row_offset, tokens, best, partials, ticket);
+        if (rc != QWEN36_STATUS_SUCCESS) return rc;
+        return launch_scan(lm_head_gemv_kernel<N, FUSED, true, true>, grid, static_cast<size_t>(N) * cols * 4, Gate{gate.redo, nullptr}, w,
+                           scales, x, y, rows, static_cast<uint32_t>(cols), row_offset, tokens, best, partials, ticket);
       }
-      return launch_gemv_x<N, FUSED, true>(w, scales, x, y, rows, cols, row_offset, tokens, best, partials, ticket, grid);
+      return launch_gemv_x<N, FUSED, true>(w, scales, x, y, rows, cols, row_offset, tokens, best, partials, ticket, grid, gate);
     }
   }
-  return launch_gemv_x<N, FUSED, false>(w, scales, x, y, rows, cols, row_offset, tokens, best, partials, ticket, grid);
+  return launch_gemv_x<N, FUSED, false>(w, scales, x, y, rows, cols, row_offset, tokens, best, partials, ticket, grid, gate);
 }
 
 // Persistent grid: enough CTAs to fill the GPU, never more than there is work.
@@ -1100,11 +1151,11 @@ unsigned gemv_grid(size_t rows, size_t n, size_t cols) {
 template <bool FUSED>
 int launch_gemv(size_t n, const uint8_t *w, const float *scales, const __nv_bfloat16 *x, __nv_bfloat16 *y,
                 size_t rows, size_t cols, uint32_t row_offset, uint32_t *tokens, float *best, float2 *partials,
-                unsigned *ticket, size_t slots) {
+                unsigned *ticket, size_t slots, const Gate &gate) {
   unsigned grid = gemv_grid(rows, n, cols);
   if (FUSED && grid > slots) grid = static_cast<unsigned>(slots);
 #define Q36_CASE(NN) \
-  case NN: return launch_gemv_n<NN, FUSED>(w, scales, x, y, rows, cols, row_offset, tokens, best, partials, ticket, grid, slots);
+  case NN: return launch_gemv_n<NN, FUSED>(w, scales, x, y, rows, cols, row_offset, tokens, best, partials, ticket, grid, slots, gate);
   switch (n) {
     Q36_CASE(1) Q36_CASE(2) Q36_CASE(3) Q36_CASE(4) Q36_CASE(5) Q36_CASE(6) Q36_CASE(7) Q36_CASE(8)
     Q36_CASE(9) Q36_CASE(10) Q36_CASE(11) Q36_CASE(12) Q36_CASE(13) Q36_CASE(14) Q36_CASE(15) Q36_CASE(16)
@@ -1146,7 +1197,7 @@ extern "C" int qwen36_lm_head_fp8_gemv(const qwen36_lm_head_fp8_gemv_spec_t *spe
     const int rc = launch_gemv<false>(nt, as_ptr<const uint8_t>(spec->weight_e4m3), as_ptr<const float>(spec->row_scales_f32),
                                       as_ptr<const __nv_bfloat16>(spec->input_bf16) + t0 * spec->cols,
                                       as_ptr<__nv_bfloat16>(spec->output_bf16) + t0 * spec->rows, spec->rows, spec->cols, 0u,
-                                      nullptr, nullptr, nullptr, nullptr, 0);
+                                      nullptr, nullptr, nullptr, nullptr, 0, Gate{nullptr, nullptr});
     if (rc != QWEN36_STATUS_SUCCESS) return rc;
   }
   return QWEN36_STATUS_SUCCESS;
@@ -1169,31 +1220,29 @@ extern "C" int qwen36_lm_head_fp8_gemv_argmax(const qwen36_lm_head_fp8_argmax_sp
   // the ticket (it is back at zero when a launch ends) and the winners' slots
   for (size_t t0 = 0; t0 < spec->n; t0 += kChunkTokens) {
     const size_t nt = spec->n - t0 < kChunkTokens ? spec->n - t0 : kChunkTokens;
-    float *best = as_ptr<float>(spec->best_value_f32);
+    const uint8_t *w = as_ptr<const uint8_t>(spec->weight_e4m3);
+    const float *scales = as_ptr<const float>(spec->row_scales_f32);
+    const __nv_bfloat16 *x = as_ptr<const __nv_bfloat16>(spec->input_bf16) + t0 * spec->cols;
+    uint32_t *tokens = as_ptr<uint32_t>(spec->output_token_u32) + t0;
+    float *best = spec->best_value_f32.ptr == 0 ? nullptr : as_ptr<float>(spec->best_value_f32) + t0;
+    unsigned *ticket = as_ptr<unsigned>(spec->workspace);
+    float2 *partials = reinterpret_cast<float2 *>(static_cast<uintptr_t>(spec->workspace.ptr + 16));
+    Gate gate{nullptr, nullptr};
     if (bound_route(spec->rows, spec->cols, nt, spec->workspace_bytes, spec->n)) {
+      uint8_t *scratch = as_ptr<uint8_t>(spec->workspace) + winners_bytes(spec->n);
       int rc = QWEN36_STATUS_INVALID_ARGUMENT;
 #define Q36_BOUND(NN) \
-  case NN: rc = launch_bound<NN>(as_ptr<const uint8_t>(spec->weight_e4m3), as_ptr<const float>(spec->row_scales_f32), \
-                                 as_ptr<const __nv_bfloat16>(spec->input_bf16) + t0 * spec->cols, spec->rows, spec->cols, \
-                                 spec->row_offset, as_ptr<uint32_t>(spec->output_token_u32) + t0, \
-                                 best == nullptr ? nullptr : best + t0, \
-                                 reinterpret_cast<float2 *>(static_cast<uintptr_t>(spec->workspace.ptr + 16)), \
-                                 as_ptr<unsigned>(spec->workspace), \
-                                 as_ptr<uint8_t>(spec->workspace) + winners_bytes(spec->n)); break;
+  case NN: rc = launch_bound<NN>(w, scales, x, spec->rows, spec->cols, spec->row_offset, tokens, best, partials, ticket, scratch); break;
       switch (nt) {
         Q36_BOUND(4) Q36_BOUND(5) Q36_BOUND(6) Q36_BOUND(7) Q36_BOUND(8)
         default: break;
       }
 #undef Q36_BOUND
       if (rc != QWEN36_STATUS_SUCCESS) return rc;
-      continue;
+      gate = Gate{reinterpret_cast<unsigned *>(scratch) + 1, ticket + 1};
     }
-    const int rc = launch_gemv<true>(nt, as_ptr<const uint8_t>(spec->weight_e4m3), as_ptr<const float>(spec->row_scales_f32),
-                                     as_ptr<const __nv_bfloat16>(spec->input_bf16) + t0 * spec->cols, nullptr, spec->rows,
-                                     spec->cols, spec->row_offset, as_ptr<uint32_t>(spec->output_token_u32) + t0,
-                                     best == nullptr ? nullptr : best + t0,
-                                     reinterpret_cast<float2 *>(static_cast<uintptr_t>(spec->workspace.ptr + 16)),
-                                     as_ptr<unsigned>(spec->workspace), slots);
+    const int rc = launch_gemv<true>(nt, w, scales, x, nullptr, spec->rows, spec->cols, spec->row_offset, tokens, best, partials,
+                                     ticket, slots, gate);
     if (rc != QWEN36_STATUS_SUCCESS) return rc;
   }
   return QWEN36_STATUS_SUCCESS;

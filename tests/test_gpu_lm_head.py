@@ -195,3 +195,30 @@ def test_fused_argmax_stays_inside_a_small_workspace(backend, n):
     tok, _ = backend.lm_head_fp8_gemv_argmax(to_dev(w), to_dev(s), to_dev(x), buf[: 16 + 5 * 8 * n])
     assert np.array_equal(tok.cpu().numpy().astype(np.uint32), orc.argmax_rows(orc.lm_head_fp8_gemv(w, s, x)))
     assert bool((buf[16 + 5 * 8 * n:] == 0xA5).all())
+
+
+@pytest.mark.parametrize("n,cols", [(4, 2176), (8, 2176), (5, 5120), (7, 128)])
+def test_exact_scan_takes_over_where_bounds_do_not_help(backend, n, cols):
+    """Equal rows, a zeroed weight, a block of near-copies of the best row, an infinity: the exact scan behind the bounds does the
+    work, and the next call with the same workspace is an ordinary one again.  Tokens and values equal the oracle's."""
+    rows = BOUND_ROWS[cols]
+    rng = np.random.default_rng(n + cols)
+    plain, s = synth.lm_head_weight(rng, rows, cols)
+    x = synth.activations(rng, n, cols)
+    best = int(np.argmax(synth.bf16_bits_to_f32(orc.lm_head_fp8_gemv(plain, s, x[:1])[0])))
+    copies, copy_s = plain.copy(), s.copy()
+    first = rows // 3
+    copies[first:first + rows // 3], copy_s[first:first + rows // 3] = plain[best], s[best]
+    copies[first:first + rows // 3, 7] ^= rng.integers(0, 2, rows // 3).astype(np.uint8)      # ties and last bits
+    x_inf = x.copy(); x_inf[n - 1, 5] = 0x7F80
+    ws = backend.lm_head_argmax_workspace(rows, n, "cuda")
+    redo = ws[16 + 148 * 4 * 8 * n + 4:][:4].view(torch.int32)
+    for w, sc, act, scanned in ((plain, s, x, 0), (np.broadcast_to(plain[3], plain.shape), np.full_like(s, s[3]), x, 1), (plain, s, x, 0),
+                                (np.zeros_like(plain), s, x, 1), (copies, copy_s, x, 1), (plain, s, x_inf, 1), (plain, s, x, 0)):
+        tok, value = backend.lm_head_fp8_gemv_argmax(to_dev(np.ascontiguousarray(w)), to_dev(sc), to_dev(act), ws)
+        logits = orc.lm_head_fp8_gemv(np.ascontiguousarray(w), sc, act)
+        want = orc.argmax_rows(logits)
+        values = synth.bf16_bits_to_f32(logits[np.arange(n), want])
+        assert np.array_equal(tok.cpu().numpy().astype(np.uint32), want)
+        assert np.array_equal(value.cpu().numpy(), np.where(np.isnan(values), -np.inf, values))
+        assert redo.item() == scanned and int(ws[:16].sum()) == 0
