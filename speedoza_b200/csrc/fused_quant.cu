@@ -327,7 +327,7 @@ __device__ __noinline__ uint32_t swiglu_exact_word(uint4 gv, uint4 uv, float ds)
   const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w}, uw[4] = {uv.x, uv.y, uv.z, uv.w};
   const float rcp = __frcp_rn(ds);
   uint32_t word = 0u;
-#pragma unroll 1
+#pragma unroll
   for (int i = 0; i < 4; ++i) {
     const float x0 = swiglu_value(low_half(gw[i]), low_half(uw[i])), x1 = swiglu_value(high_half(gw[i]), high_half(uw[i]));
     float e0 = __fmul_rn(x0, rcp), e1 = __fmul_rn(x1, rcp);
@@ -355,13 +355,14 @@ __device__ __forceinline__ uint32_t e2m1x8(const float (&q)[8]) {
 // (SwiGLU kernel, then qwen36_nvfp4_quantize_rows) is never written or read back.  Row r of the
 // output is what swiglu_nvfp4_quantize_kernel gives for row r alone (same expressions in float32,
 // no bf16 round trip), its scale bytes at the tiled position of (group, r).
-// Sixteen expf, sixteen divisions and the bookkeeping of their special cases per group made a kernel that evaluates the
-// expressions issue-bound (51 instruction slots per value).  Their last bits only matter where a result sits next to a
-// rounding boundary of the scale or of a code, so swiglu_estimate decides: eight codes are taken twice, from quotients
+// Sixteen expf, sixteen divisions and the bookkeeping of their special cases per group make a kernel that evaluates the
+// expressions (below) issue-bound: 51 instruction slots per value.  Their last bits only matter where a result sits next to a
+// rounding boundary of the scale or of a code, so swiglu_estimate decides here: eight codes are taken twice, from quotients
 // pushed up and down by 2^-16 (the estimate's error is below 2^-17, reciprocal and product add three ulps), and where the
 // two differ the eight are redone from the reference's expressions.  The same for the scale, whose group is redone when
-// 256 ulps decide, or when it holds zeros, tiny values, infinities or NaN.  (A mask on the quotients' bits that finds the
-// pairs next to a boundary, and denormal-safe ex2 / rcp, left 43 slots per value and no gain.)
+// 256 ulps decide, or when it holds tiny values, infinities or NaN; zeros are exact, have no part in the scale, and code 0.
+// (A mask on the quotients' bits that finds the pairs next to a boundary, and denormal-safe ex2 / rcp, left 43 slots per
+// value and no gain.)
 // blockDim (64, 4): two lanes share a 16-group of a row (one 16-byte load of gate and of up each), rows advance by the
 // grid with the next two rows' loads in flight.  Figures at the entry point.
 __global__ void __launch_bounds__(256, 4)
@@ -413,6 +414,14 @@ swiglu_nvfp4_quantize_rows_kernel(const __nv_bfloat16 *__restrict__ gate, const 
       asm("max.NaN.f32 %0, %0, %1;" : "+f"(amax) : "f"(fabsf(y[i])));    // a NaN must not hide: it fails the range check below
       amin = fminf(amin, fabsf(y[i]));
     }
+    if (amin < 0x1p-90f) {                                           // zeros whose factors say so are exact: not among the tiny values
+      amin = INFINITY;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if ((gw[i] & 0x7fffu) != 0u && (uw[i] & 0x7fffu) != 0u) amin = fminf(amin, fabsf(y[2 * i]));
+        if ((gw[i] & 0x7fff0000u) != 0u && (uw[i] & 0x7fff0000u) != 0u) amin = fminf(amin, fabsf(y[2 * i + 1]));
+      }
+    }
     asm("max.NaN.f32 %0, %0, %1;" : "+f"(amax) : "f"(__shfl_xor_sync(0xffffffffu, amax, 1)));
     amin = fminf(amin, __shfl_xor_sync(0xffffffffu, amin, 1));
     const float sv = __fmul_rn(amax, rcp6);
@@ -426,11 +435,13 @@ swiglu_nvfp4_quantize_rows_kernel(const __nv_bfloat16 *__restrict__ gate, const 
         const float rcp = rcp_estimate(ds), rcp_up = rcp * (1.0f + 0x1p-16f), rcp_down = rcp * (1.0f - 0x1p-16f);
         float q[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) q[i] = y[i] * rcp_down;
+        for (int i = 0; i < 8; ++i) q[i] = fmaf(y[i], rcp_down, 0.0f);      // a zero of either sign becomes +0, code 0
         word = e2m1x8(q);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) q[i] = y[i] * rcp_up;
+        for (int i = 0; i < 8; ++i) q[i] = fmaf(y[i], rcp_up, 0.0f);
         if (word != e2m1x8(q)) word = swiglu_exact_word(make_uint4(gw[0], gw[1], gw[2], gw[3]), make_uint4(uw[0], uw[1], uw[2], uw[3]), ds);
+      } else if (amax == 0.0f && amin == INFINITY) {                 // sixteen exact zeros (a row of padding): scale 1.0, codes 0
+        sf_code = 0x38u;
       } else {
         const uint2 exact = swiglu_exact_half_group(gp - half * 8u, upp - half * 8u, half, g, six_g, rcp6);
         word = exact.x;
@@ -455,6 +466,79 @@ swiglu_nvfp4_quantize_rows_kernel(const __nv_bfloat16 *__restrict__ gate, const 
   }
 }
 
+// The same with the reference's expressions for every value: a thread owns one 16-group of a row (blockDim (64, 4)), rows
+// advance by the grid with the next row's 64 bytes already in flight.
+__global__ void __launch_bounds__(256)
+swiglu_nvfp4_quantize_rows_exact_kernel(const __nv_bfloat16 *__restrict__ gate, const __nv_bfloat16 *__restrict__ up,
+                                  uint8_t *__restrict__ out_fp4, uint8_t *__restrict__ out_sf,
+                                  float *__restrict__ tensor_scale, uint32_t rows, uint32_t values, size_t stride,
+                                  float input_tensor_scale) {
+  const float g = input_tensor_scale > 0.0f ? input_tensor_scale : 1.0f;
+  const float six_g = __fmul_rn(6.0f, g), rcp6 = __frcp_rn(six_g);
+  const uint32_t groups = values >> 4, padded = (groups + 3u) & ~3u;
+  const uint32_t group = blockIdx.x * 64u + threadIdx.x;
+  const bool in_row = group < groups;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (rows < q36::kWeightRows) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0 && tensor_scale != nullptr) *tensor_scale = g;
+
+  const uint32_t row_step = gridDim.y * 4u;
+  uint32_t row = blockIdx.y * 4u + threadIdx.y;
+  uint4 ng0 = make_uint4(0u, 0u, 0u, 0u), ng1 = ng0, nu0 = ng0, nu1 = ng0;
+  if (in_row && row < rows) {
+    const size_t at = static_cast<size_t>(row) * stride + group * 16u;
+    ng0 = __ldcs(reinterpret_cast<const uint4 *>(gate + at));
+    ng1 = __ldcs(reinterpret_cast<const uint4 *>(gate + at) + 1);
+    nu0 = __ldcs(reinterpret_cast<const uint4 *>(up + at));
+    nu1 = __ldcs(reinterpret_cast<const uint4 *>(up + at) + 1);
+  }
+  for (; row < rows; row += row_step) {
+    uint32_t sf_code = 0;
+    const uint32_t gw[8] = {ng0.x, ng0.y, ng0.z, ng0.w, ng1.x, ng1.y, ng1.z, ng1.w};
+    const uint32_t uw[8] = {nu0.x, nu0.y, nu0.z, nu0.w, nu1.x, nu1.y, nu1.z, nu1.w};
+    if (in_row && row + row_step < rows) {
+      const size_t at = static_cast<size_t>(row + row_step) * stride + group * 16u;
+      ng0 = __ldcs(reinterpret_cast<const uint4 *>(gate + at));
+      ng1 = __ldcs(reinterpret_cast<const uint4 *>(gate + at) + 1);
+      nu0 = __ldcs(reinterpret_cast<const uint4 *>(up + at));
+      nu1 = __ldcs(reinterpret_cast<const uint4 *>(up + at) + 1);
+    }
+    if (in_row) {
+      float y[16];
+      float amax = 0.0f;
+      uint32_t any = 0u, smallest = 0xffffffffu;                  // smallest nonzero magnitude, as bits - 1
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const float gv = __uint_as_float((i & 1) ? (gw[i >> 1] & 0xffff0000u) : (gw[i >> 1] << 16));
+        const float uv = __uint_as_float((i & 1) ? (uw[i >> 1] & 0xffff0000u) : (uw[i >> 1] << 16));
+        const float silu = gv / (1.0f + expf(-gv));
+        y[i] = silu * uv;
+        amax = fmaxf(amax, fabsf(y[i]));
+        const uint32_t mag = __float_as_uint(y[i]) & 0x7fffffffu;
+        any |= mag;
+        smallest = min(smallest, mag - 1u);
+      }
+      uint32_t lo, hi;
+      q36::nvfp4_quantize_group(y, amax, any != 0u, smallest < 0x0f800000u, g, six_g, rcp6, lo, hi, sf_code);
+      *reinterpret_cast<uint2 *>(out_fp4 + (static_cast<size_t>(row) * (values >> 1) + group * 8u)) = make_uint2(lo, hi);
+    }
+    // the four scale bytes of a quad of groups form one word of the tiled layout (see q36::sf_offset)
+    const uint32_t lane4 = threadIdx.x & 3u;
+    uint32_t word = sf_code << (8u * lane4);
+    word |= __shfl_xor_sync(0xffffffffu, word, 1);
+    word |= __shfl_xor_sync(0xffffffffu, word, 2);
+    if (in_row) {
+      const size_t off = (static_cast<size_t>(group >> 2) + static_cast<size_t>(row >> 7) * (padded >> 2)) * 512u +
+                         (row & 31u) * 16u + ((row >> 5) & 3u) * 4u + lane4;
+      if ((group | 3u) < groups) {
+        if (lane4 == 0u) *reinterpret_cast<uint32_t *>(out_sf + off) = word;
+      } else {
+        out_sf[off] = static_cast<uint8_t>(sf_code);
+      }
+    }
+  }
+}
+
 }  // namespace
 
 extern "C" int qwen36_swiglu_nvfp4_quantize_rows(const qwen36_swiglu_nvfp4_quantize_rows_spec_t *spec) {
@@ -468,13 +552,19 @@ extern "C" int qwen36_swiglu_nvfp4_quantize_rows(const qwen36_swiglu_nvfp4_quant
       (spec->output_scale_e4m3.ptr & 3u) != 0 || spec->rows >= (1ull << 31) || spec->intermediate >= (1ull << 31))
     return QWEN36_STATUS_INVALID_ARGUMENT;
   const size_t padded = q36::round_up(spec->intermediate / 16, 4);
-  // 2048 x 17408: 57.6 us with every value from expf and a division, 47.6 us now (24.5 us of HBM time; about 30 instruction
-  // slots per value are left); 1000 x 17408 inside a block: 33.1 -> 25.5 us
-  const size_t gx = q36::div_ceil(padded, 32), row_chunks = q36::div_ceil(spec->rows, 4);
-  const size_t want = q36::div_ceil(static_cast<size_t>(q36::sm_count_current_device()) * 20, gx);
+  // Estimates decide from six million values up, where instruction slots bound the kernel, and below 16384, where few lanes ever
+  // leave them; in between a slow path that a few warps take, its instructions not yet in the cache, is what the launch waits
+  // for, and the reference's expressions throughout are the faster ones.  us back to back, expressions | estimates:
+  //   2 x 4096 2.59 | 2.36   5 x 17408 2.72 | 3.23   64 x 8704 2.85 | 3.86   200 x 17408 8.4 | 9.2   300 x 17408 11.6 | 12.2
+  //   2048 x 4096 17.2 | 16.8   1000 x 17408 31.6 | 26.8   2048 x 17408 56.0 | 46.4 (24.5 us of HBM time)
+  // With a tenth of the inputs zero the estimates take 52.7 us at 2048 x 17408, the expressions 138.
+  const size_t count = spec->rows * spec->intermediate;
+  const bool exact = count >= (16u << 10) && count < (6u << 20);
+  const size_t gx = q36::div_ceil(padded, exact ? 64 : 32), row_chunks = q36::div_ceil(spec->rows, 4);
+  const size_t want = q36::div_ceil(static_cast<size_t>(q36::sm_count_current_device()) * (exact ? 24 : 20), gx);
   const dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(row_chunks < want ? row_chunks : want));
   return q36::cuda_status(q36::launch_after_previous(
-      swiglu_nvfp4_quantize_rows_kernel, grid, dim3(64, 4), size_t{0}, q36::stream(),
+      exact ? swiglu_nvfp4_quantize_rows_exact_kernel : swiglu_nvfp4_quantize_rows_kernel, grid, dim3(64, 4), size_t{0}, q36::stream(),
       as_ptr<const __nv_bfloat16>(spec->gate_bf16), as_ptr<const __nv_bfloat16>(spec->up_bf16),
       as_ptr<uint8_t>(spec->output_fp4), as_ptr<uint8_t>(spec->output_scale_e4m3),
       as_ptr<float>(spec->output_tensor_scale_f32), static_cast<uint32_t>(spec->rows),

@@ -122,7 +122,7 @@ def _special_rows(rng, rows, n):
     return gate, up
 
 
-@pytest.mark.parametrize("rows,n,its", [(5, 17408, 0.37), (130, 1088, 0.0), (3, 16, 1.25), (257, 80, 0.0)])
+@pytest.mark.parametrize("rows,n,its", [(5, 17408, 0.37), (130, 1088, 0.0), (3, 16, 1.25), (257, 80, 0.0), (9, 1088, 0.37), (5, 144, 0.0)])
 def test_swiglu_rows_equal_the_single_vector_entry_row_by_row(backend, rows, n, its):
     """qwen36_swiglu_nvfp4_quantize_rows: every row's code bytes and scale bytes are those of
     qwen36_swiglu_nvfp4_quantize on that row (itself byte-identical to the reference's kernel), also
@@ -197,9 +197,9 @@ def test_swiglu_rows_argument_checks(backend):
 @pytest.mark.parametrize("gate_std,up_std,its,bits", [(2.0, 1.0, 0.0, 8), (2.0, 1.0, 0.11, 8), (12.0, 3.0, 0.37, 3), (60.0, 1e4, 1.25, 8),
                                                       (0.01, 1e-3, 0.0, 2), (0.5, 1.0, 1e-6, 8), (1.0, 30.0, 300.0, 4)])
 def test_swiglu_rows_every_byte_of_a_large_block(backend, gate_std, up_std, its, bits):
-    """1.6 M values per distribution (few mantissa bits: quotients near ties; wide gates: results down to zero), every code
-    and scale byte against the single-vector entry on the same values laid out as one vector."""
-    rows, n = 384, 4112
+    """6.6 M values per distribution (few mantissa bits: quotients near ties; wide gates: results down to zero; zeros of both
+    signs), every code and scale byte against the single-vector entry on the same values laid out as one vector."""
+    rows, n = 1600, 4112
     gen = torch.Generator(device="cuda").manual_seed(int(gate_std * 100) + bits)
     def block(std):
         x = (torch.randn((rows, n), generator=gen, device="cuda") * std).to(torch.bfloat16)
@@ -207,6 +207,8 @@ def test_swiglu_rows_every_byte_of_a_large_block(backend, gate_std, up_std, its,
     gate, up = block(gate_std), block(up_std)
     gate[5] = 0
     gate[7, ::3] = 30.0                                   # silu(30) = 30
+    gate[9:19, ::5] = 0.0; up[9:19, 1::7] = -0.0          # zeros among other values
+    up[20:24] = -0.0; up[22, ::31] = 2.0 ** -130          # rows of zeros, one with tiny values in it
     fp4, sf, _ = backend.swiglu_nvfp4_quantize_rows(gate, up, its)
     f1, s1, _ = backend.swiglu_nvfp4_quantize(gate.view(-1), up.view(-1), its)
     assert torch.equal(fp4.view(-1), f1)
