@@ -24,7 +24,7 @@
 // the splits (attention_flash_splitk.cu:139-149).  Decode: split s = timesteps [s * block, (s + 1)
 // * block) cut at position + 1; timestep == position is the not yet cached k_bf16 / v_bf16 row.
 #include "common.cuh"
-#include "kv_split.cuh"
+#include "launch.cuh"
 #include "lse_merge.cuh"
 
 #include <cuda_fp16.h>

@@ -17,7 +17,7 @@
 // fetches its norm weights, which are model state) while the kernel ahead drains, and lets the
 // kernel behind (a GEMV that streams its weights before it needs this output) take its seats at once.
 #include "common.cuh"
-#include "kv_split.cuh"
+#include "launch.cuh"
 #include "nvfp4_quant_group.cuh"
 
 namespace {

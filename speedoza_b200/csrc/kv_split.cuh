@@ -3,6 +3,8 @@
 // helpers of the shared-memory staged forms, and the CTA epilogue that merges the eight warps'
 // running softmax states into one (m, l, o) partial per q head.
 #pragma once
+#include "launch.cuh"
+
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -11,32 +13,6 @@ namespace q36 {
 
 constexpr int kSplitThreads = 256;
 constexpr int kSplitWarps = kSplitThreads / 32;
-
-// Launch with programmatic stream serialisation: the grid may take its seats while the previous
-// kernel in the stream drains.  The kernel must execute griddepcontrol.wait before it touches
-// anything an earlier kernel may have written (and before it overwrites anything one may still read).
-template <typename... KArgs, typename... Args>
-inline cudaError_t launch_after_previous(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem_bytes,
-                                         cudaStream_t stream, Args... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem_bytes;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
-}
-
-// Asks L2 for a piece of memory (16-byte aligned, a multiple of 16 bytes).  Reads nothing, so it may run before
-// griddepcontrol.wait: a kernel that took its seat while the one ahead drains fills L2 with the cache rows it will need,
-// whoever may still be writing one of them.
-__device__ __forceinline__ void prefetch_l2(const void *p, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
 
 __device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                         uint32_t b1) {

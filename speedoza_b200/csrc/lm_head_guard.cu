@@ -12,7 +12,7 @@
 // ONE pass over the 2.5 GB weight for all rows that still need it (the reference re-reads the
 // weight once per row), with the activations staged as float32 in shared memory.
 #include "common.cuh"
-#include "kv_split.cuh"
+#include "launch.cuh"
 
 #include <math.h>
 

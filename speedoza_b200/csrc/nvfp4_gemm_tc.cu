@@ -24,7 +24,7 @@
 //
 // Every mbarrier wait is bounded; a wait that gives up sets g_gemm_error, and all roles fall
 // through to the common exit where TMEM is released.
-#include "kv_split.cuh"
+#include "launch.cuh"
 #include "nvfp4_gemm_tc.cuh"
 
 #include <atomic>
@@ -162,11 +162,6 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
                : "r"(taddr));
 }
 
-// L2 prefetch of a contiguous piece (16-byte aligned, a multiple of 16 bytes)
-__device__ __forceinline__ void bulk_prefetch(const void *src, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
-}
-
 template <uint32_t BN> struct Cfg {
   static constexpr uint32_t kSfbTiles = (BN + 127) / 128;              // 512-byte scale tiles per K=64 for B
   static constexpr uint32_t kBRows = BN < 8 ? 8 : BN;
@@ -242,7 +237,7 @@ nvfp4_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   auto prefetch_one = [&]() {
     if (pf_tile >= tiles) return;
     tma_prefetch_2d(&map_a, pf_kb * kBKBytes, (pf_tile / n_blocks) * kBM);
-    bulk_prefetch(a_sf + (static_cast<size_t>(pf_tile / n_blocks) * sf_tiles_per_block + pf_kb * 4u) * 512u, 2048u);
+    q36::prefetch_l2(a_sf + (static_cast<size_t>(pf_tile / n_blocks) * sf_tiles_per_block + pf_kb * 4u) * 512u, 2048u);
     if (++pf_kb == k_blocks) { pf_kb = 0; pf_tile += gridDim.x; }
   };
   // Launched while the kernel ahead drains: nothing may be read before that kernel is done (a caller may have
@@ -1171,7 +1166,7 @@ nvfp4_gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   if (threadIdx.x == 0) {
     for (uint32_t kb = kb_begin; kb < kb_end && kb < kb_begin + C::kStages + 2u; ++kb) {
       tma_prefetch_2d(&map_a, kb * kBKBytes, mb * kBM);
-      bulk_prefetch(a_sf + (static_cast<size_t>(mb) * sf_tiles_per_block + kb * 4u) * 512u, 2048u);
+      q36::prefetch_l2(a_sf + (static_cast<size_t>(mb) * sf_tiles_per_block + kb * 4u) * 512u, 2048u);
     }
   }
   __syncwarp();

@@ -7,7 +7,7 @@
 // 704-761): IEEE float32 division by the decoded scale, E2M1 ties toward zero,
 // UE4M3 ties down.
 #include "common.cuh"
-#include "kv_split.cuh"
+#include "launch.cuh"
 #include "nvfp4_quant_group.cuh"
 
 #include <atomic>
