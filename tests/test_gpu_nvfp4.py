@@ -549,3 +549,27 @@ def test_w4a4_gemm_stream_k_under_graph_replay(backend):
         backend.lib.qwen36_nvfp4_gemm_stream_k(0)
         backend.sync_stream()
     assert backend.lib.qwen36_nvfp4_gemm_last_error() == 0
+
+
+@pytest.mark.parametrize("m,n,k,stream_k", [(1280, 8192, 17408, 2), (5120, 1000, 17408, 0), (1280, 600, 5120, 1)])
+def test_pair_gemm_gives_the_same_bits_on_every_launch(backend, m, n, k, stream_k):
+    """Three hundred launches behind one another against the first, compared on the device.  The CTA-pair kernel's scale
+    ring once let a copier run a phase ahead of a late load: one wrong tile in some ten launches of the first shape."""
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    packed, sf_rm = synth.nvfp4_weight_device(gen, m, k, "cuda")
+    sfa = backend.nvfp4_retile_scales(sf_rm)
+    fp4, sfb, ts = backend.nvfp4_quantize_rows(torch.randn((n, k), generator=gen, device="cuda").to(torch.bfloat16), 0.37)
+    alpha = float(np.float32(synth.WEIGHT_GLOBAL_SCALE) * np.float32(ts.item()))
+    out = torch.empty((4, n, m), dtype=torch.bfloat16, device="cuda")
+    wrong = torch.zeros((), dtype=torch.int64, device="cuda")
+    try:
+        backend.lib.qwen36_nvfp4_gemm_stream_k(stream_k)
+        first = backend.nvfp4_gemm(packed, sfa, fp4, sfb, alpha, m, n, k).clone()
+        torch.cuda.synchronize()
+        for _ in range(75):
+            for o in out:
+                backend.nvfp4_gemm(packed, sfa, fp4, sfb, alpha, m, n, k, o)
+            wrong += (out.view(torch.int16) != first.view(torch.int16)).sum()
+    finally:
+        backend.lib.qwen36_nvfp4_gemm_stream_k(0)
+    assert wrong.item() == 0 and backend.lib.qwen36_nvfp4_gemm_last_error() == 0
