@@ -222,9 +222,10 @@ struct Gate {
   const unsigned *redo;
   unsigned *counter;
 };
+template <bool FOLLOWED>                                           // by the other of two scans, which may take its seats: it waits first
 __device__ __forceinline__ bool gate_closed(const Gate gate) {
   if (gate.redo == nullptr) return false;
-  if (gate.counter != nullptr) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the other scan, which waits first
+  if (FOLLOWED) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (gate.counter != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *gate.counter = 0u;
   return __ldcg(gate.redo) == 0u;
@@ -240,7 +241,7 @@ lm_head_gemv_kernel(const uint8_t *__restrict__ weight, const float *__restrict_
                     float *__restrict__ out_best, float2 *__restrict__ partials,
                     unsigned *__restrict__ ticket, const Gate gate) {
   constexpr int R = RowsPerWarp<N, XF32>::value;
-  if (FUSED && gate_closed(gate)) return;
+  if (FUSED && gate_closed<false>(gate)) return;
   extern __shared__ __align__(16) uint8_t smem[];
   uint4 *xs = reinterpret_cast<uint4 *>(smem);        // N * cols bf16, swizzled chunks
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -384,7 +385,7 @@ lm_head_gemv_f16_kernel(const uint8_t *__restrict__ weight, const float *__restr
                         float *__restrict__ out_best, float2 *__restrict__ partials,
                         unsigned *__restrict__ ticket, const Gate gate) {
   constexpr int R = kF16Rows;
-  if (FUSED && gate_closed(gate)) return;
+  if (FUSED && gate_closed<true>(gate)) return;
   constexpr int S = F16Ring<N>::kStages;
   extern __shared__ __align__(16) uint8_t smem[];
   uint4 *xs = reinterpret_cast<uint4 *>(smem);        // N * cols float16, swizzled 16-byte chunks
