@@ -263,7 +263,12 @@ int qwen36_decode_nvfp4_gemv(const qwen36_nvfp4_gemm_spec_t *spec);
  * kept for linkage, has no effect. */
 void qwen36_nvfp4_chunk_gemv_set_mtile(int mtile);
 
-/* Replaces qwen36_nvfp4_matvec (kernels-cuda/ops.cu:547-639,1155-1180). */
+/* Replaces qwen36_nvfp4_matvec (kernels-cuda/ops.cu:547-639,1155-1180).  The
+ * one-token kernels (this one, its group form, qwen36_decode_nvfp4_gemv and
+ * qwen36_nvfp4_gemm at n = 1) start while the call ahead on the stream drains
+ * and read weights, scales and tensor scale before they wait for it.  What this
+ * library's quantisers write is complete by then; another kernel of this
+ * library that writes a weight must not be the call directly ahead. */
 int qwen36_nvfp4_matvec(const qwen36_nvfp4_matvec_spec_t *spec);
 
 /* Additive: `count` (1..4) GEMVs that share input_bf16 and in_features, as ONE launch whose work
@@ -377,7 +382,9 @@ typedef struct {                         /* qwen36_fp4.h:151-183 */
  * says: [q_heads, decode_n_splits, head_dim] and 2 x [q_heads, decode_n_splits]);
  * how many of them are used and which rows each one takes is this library's
  * choice, so split_timesteps_per_block is only validated (>= 64 or 0).  Without
- * the buffers one CTA per q head walks the whole context.  TurboQuant3 / 3.5
+ * the buffers one CTA per q head walks the whole context in float32; with them
+ * the softmax weights (and over an FP8 cache q) are multiplied as 16-bit values,
+ * in two terms where the context takes the one-launch form.  TurboQuant3 / 3.5
  * caches (dtype 2 / 3) return QWEN36_STATUS_NOT_IMPLEMENTED. */
 int qwen36_attention_decode(const qwen36_attention_decode_spec_t *spec);
 
