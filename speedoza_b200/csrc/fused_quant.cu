@@ -470,9 +470,9 @@ swiglu_nvfp4_quantize_rows_kernel(const __nv_bfloat16 *__restrict__ gate, const 
 // advance by the grid with the next row's 64 bytes already in flight.
 __global__ void __launch_bounds__(256)
 swiglu_nvfp4_quantize_rows_exact_kernel(const __nv_bfloat16 *__restrict__ gate, const __nv_bfloat16 *__restrict__ up,
-                                  uint8_t *__restrict__ out_fp4, uint8_t *__restrict__ out_sf,
-                                  float *__restrict__ tensor_scale, uint32_t rows, uint32_t values, size_t stride,
-                                  float input_tensor_scale) {
+                                        uint8_t *__restrict__ out_fp4, uint8_t *__restrict__ out_sf,
+                                        float *__restrict__ tensor_scale, uint32_t rows, uint32_t values, size_t stride,
+                                        float input_tensor_scale) {
   const float g = input_tensor_scale > 0.0f ? input_tensor_scale : 1.0f;
   const float six_g = __fmul_rn(6.0f, g), rcp6 = __frcp_rn(six_g);
   const uint32_t groups = values >> 4, padded = (groups + 3u) & ~3u;
