@@ -702,7 +702,7 @@ decode_split_bf16_mma_kernel(const __nv_bfloat16 *__restrict__ q, const __nv_bfl
 // dims, one cluster barrier later every CTA finishes 256 / cluster dims of every head, the current token added in float32,
 // and appends them to the cache.  Operand formats are those of the split kernels (float16 for FP8, bfloat16 for BF16),
 // float32 everywhere else.  Sixteen warps: with eight, scores and P V took long enough to show from 2000 tokens up
-// (FP8 4097: 9.0 us against 8.5).  The second terms cost 2 - 3 % (FP8 4097: 8.7 -> 8.9, BF16 600: 5.0 -> 5.1).  Measured
+// (FP8 4097: 9.0 us against 8.5).  The second terms cost 2 - 3 %.  Measured
 // figures are at one_launch_cluster.
 template <bool FP8> struct OneLaunch {
   static constexpr uint32_t kRowBytes = FP8 ? 256 : 512;
@@ -742,11 +742,20 @@ decode_one_launch_kernel(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat1
   const uint32_t ctas = gridDim.x, rank = blockIdx.x, kvh = blockIdx.y, head0 = kvh * G;
   const uint32_t dims = D / ctas;                                 // dims of every head that this CTA finishes
   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // "this CTA runs": waited for before the first remote store
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const size_t begin = min(position, static_cast<size_t>(T) * rank);
   const uint32_t count = static_cast<uint32_t>(min(position - begin, static_cast<size_t>(T)));
   const uint32_t groups = (count + 15) / 16;
+  {
+    // while the kernel ahead drains, L2 is asked for the cluster's rows: they are contiguous over the kv heads, of which
+    // every CTA of this rank takes an equal part (4 KB a request: a request per cache row took longer to issue than it
+    // saved; FP8 4097 8.68 -> 8.57 us, BF16 2000 7.34 -> 7.17)
+    const uint32_t first = count * kvh / kv_heads, last = count * (kvh + 1) / kv_heads;
+    const size_t at = (begin + first) * kv_heads * RB;
+    q36::prefetch_l2_span(static_cast<const uint8_t *>(cache_k) + at, (last - first) * kv_heads * RB, threadIdx.x);
+    q36::prefetch_l2_span(static_cast<const uint8_t *>(cache_v) + at, (last - first) * kv_heads * RB, kOneThreads - 1 - threadIdx.x);
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   // all of K, then all of V; rows past the end of the share are zero-filled.  Chunks are swizzled on the way in as in
   // the split kernels: K chunk c of row r at c ^ 4 (r & 1), V chunk c of row r at c ^ 2 ((r / 2) & 3).
@@ -790,6 +799,14 @@ decode_one_launch_kernel(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat1
                  __bfloat162float(k_new[static_cast<size_t>(kvh) * D + lane + 32 * j]), dot);
     for (int off = 16; off > 0; off >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, off);
     if (lane == 0) s_new[warp] = dot * sm_scale;
+  }
+  // What this thread finishes at the end: dim `fin_dim` of head `fin_head`, with the current token's values.  Fetched here:
+  // behind the last barrier their latency was a third of a microsecond (FP8 4097 8.94 -> 8.68 us, BF16 2000 7.45 -> 7.34).
+  const uint32_t fin_head = threadIdx.x / dims, fin_dd = threadIdx.x % dims, fin_dim = rank * dims + fin_dd;
+  __nv_bfloat16 kb = __float2bfloat16(0.f), vb = kb;
+  if (fin_head < G) {
+    kb = k_new[static_cast<size_t>(kvh) * D + fin_dim];
+    vb = v_new[static_cast<size_t>(kvh) * D + fin_dim];
   }
   cp_async_wait<1>();
   __syncthreads();
@@ -958,24 +975,24 @@ decode_one_launch_kernel(const __nv_bfloat16 *__restrict__ q, const __nv_bfloat1
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 
-  for (uint32_t i = threadIdx.x; i < G * dims; i += kOneThreads) {
-    const uint32_t head = i / dims, dd = i % dims, dim = rank * dims + dd;
-    const __nv_bfloat16 kb = k_new[static_cast<size_t>(kvh) * D + dim], vb = v_new[static_cast<size_t>(kvh) * D + dim];
-    const float s = s_new[head];
+  static_assert(G * (D / 8) <= static_cast<uint32_t>(kOneThreads), "one output per thread");   // clusters of eight CTAs or more
+  if (fin_head < G) {
+    const float s = s_new[fin_head];
     float top = s;
-    for (uint32_t c = 0; c < ctas; ++c) top = fmaxf(top, s_ml[c][head].x);
+#pragma unroll 4
+    for (uint32_t c = 0; c < ctas; ++c) top = fmaxf(top, s_ml[c][fin_head].x);
     const float p = exp2f(s - top);
     float den = p, acc = p * __bfloat162float(vb);
 #pragma unroll 4
     for (uint32_t c = 0; c < ctas; ++c) {
-      const float2 ml = s_ml[c][head];
+      const float2 ml = s_ml[c][fin_head];
       const float w = ml.x == -INFINITY ? 0.f : exp2f(ml.x - top);
       den = fmaf(w, ml.y, den);
-      acc = fmaf(w, s_slices[(2 * c * G + head) * dims + dd] + s_slices[((2 * c + 1) * G + head) * dims + dd], acc);
+      acc = fmaf(w, s_slices[(2 * c * G + fin_head) * dims + fin_dd] + s_slices[((2 * c + 1) * G + fin_head) * dims + fin_dd], acc);
     }
-    out[static_cast<size_t>(head0 + head) * D + dim] = __float2bfloat16(__fdiv_rn(acc, den));
-    if (head == 0) {
-      const size_t at = (position * kv_heads + kvh) * D + dim;
+    out[static_cast<size_t>(head0 + fin_head) * D + fin_dim] = __float2bfloat16(__fdiv_rn(acc, den));
+    if (fin_head == 0) {
+      const size_t at = (position * kv_heads + kvh) * D + fin_dim;
       if (FP8) {
         static_cast<uint8_t *>(cache_k)[at] = static_cast<uint8_t>(kv_f32_to_e4m3(__bfloat162float(kb)));
         static_cast<uint8_t *>(cache_v)[at] = static_cast<uint8_t>(kv_f32_to_e4m3(__bfloat162float(vb)));

@@ -31,4 +31,11 @@ __device__ __forceinline__ void prefetch_l2(const void *p, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
+// A contiguous span, a piece of 4 KB per thread: few requests, so that a kernel that is only seated for a microsecond gets
+// them all out.
+__device__ __forceinline__ void prefetch_l2_span(const uint8_t *p, uint32_t bytes, uint32_t thread) {
+  constexpr uint32_t kPiece = 4096;
+  if (thread < (bytes + kPiece - 1) / kPiece) prefetch_l2(p + thread * kPiece, min(kPiece, bytes - thread * kPiece));
+}
+
 }  // namespace q36
