@@ -545,7 +545,7 @@ bf16_argmax_fast_kernel(const __nv_bfloat16 *__restrict__ input, const __nv_bflo
 }
 
 // Keys of the rows back to zero: a kernel and not a memset, which would be one more full stop between the launches of a chain
-// that usually has nothing to do.  All four launches overlap the end of the one ahead: FP8 logits, top-8 guard and this call on 248320 x
+// that usually has nothing to do.  All three launches overlap the end of the one ahead: FP8 logits, top-8 guard and this call on 248320 x
 // 5120, one certified row, 236.4 -> 231.6 us; with the row redone 694 -> 689.
 __global__ void bf16_argmax_clear_kernel(unsigned long long *__restrict__ best_keys, size_t rows) {
   asm volatile("griddepcontrol.wait;" ::: "memory");               // launched with programmatic stream serialisation

@@ -1386,16 +1386,16 @@ bool make_scale_map(CUtensorMap *map, uint64_t ptr, uint64_t tiles) {
   return cached_map(key, map, build_scale_map);
 }
 
-// Pairs of CTAs of `kernel` that the current device can host at once (asked once per kernel and device).
-int max_active_pairs(const void *kernel, const cudaLaunchConfig_t *cfg) {
+// Clusters of `size` CTAs of `kernel` that the current device can host at once (asked once per kernel, size and device).
+int max_active_clusters(const void *kernel, uint32_t size, const cudaLaunchConfig_t *cfg) {
   static std::mutex mu;
-  static std::vector<std::tuple<const void *, int, int>> known;
+  static std::vector<std::tuple<const void *, uint32_t, int, int>> known;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
   {
     std::lock_guard<std::mutex> lock(mu);
     for (const auto &e : known)
-      if (std::get<0>(e) == kernel && std::get<1>(e) == dev) return std::get<2>(e);
+      if (std::get<0>(e) == kernel && std::get<1>(e) == size && std::get<2>(e) == dev) return std::get<3>(e);
   }
   int v = 0;
   if (cudaOccupancyMaxActiveClusters(&v, kernel, cfg) != cudaSuccess) {
@@ -1403,7 +1403,7 @@ int max_active_pairs(const void *kernel, const cudaLaunchConfig_t *cfg) {
     v = 0;
   }
   std::lock_guard<std::mutex> lock(mu);
-  known.emplace_back(kernel, dev, v);
+  known.emplace_back(kernel, size, dev, v);
   return v;
 }
 
@@ -1434,7 +1434,7 @@ int launch_pair(const qwen36_nvfp4_gemm_spec_t *s, float alpha) {
   cfg.numAttrs = 1;
   // The grid is persistent with a static tile stride, so it must never exceed the number of
   // pairs the device can host at the same time (some SMs may have no free partner).
-  const int max_pairs = max_active_pairs(reinterpret_cast<const void *>(nvfp4_gemm_pair_kernel), &cfg);
+  const int max_pairs = max_active_clusters(reinterpret_cast<const void *>(nvfp4_gemm_pair_kernel), 2u, &cfg);
   if (max_pairs <= 0) return QWEN36_STATUS_NOT_IMPLEMENTED;
   const uint32_t pairs = tiles < static_cast<uint32_t>(max_pairs) ? tiles : static_cast<uint32_t>(max_pairs);
   cfg.gridDim = dim3(pairs * 2u);
@@ -1504,7 +1504,7 @@ int launch_pair6(const qwen36_nvfp4_gemm_spec_t *s, float alpha) {
   if (q36::ensure_dynamic_smem(reinterpret_cast<const void *>(nvfp4_gemm_pair6_kernel<false>), static_cast<int>(P::kSmemBytes)) !=
       cudaSuccess)
     return QWEN36_STATUS_CUDA_ERROR;
-  const int max_pairs = max_active_pairs(reinterpret_cast<const void *>(nvfp4_gemm_pair6_kernel<false>), &cfg);
+  const int max_pairs = max_active_clusters(reinterpret_cast<const void *>(nvfp4_gemm_pair6_kernel<false>), 2u, &cfg);
   if (max_pairs <= 0) return QWEN36_STATUS_NOT_IMPLEMENTED;
   const uint32_t all = static_cast<uint32_t>(max_pairs);
   const uint64_t units = static_cast<uint64_t>(tiles) * (s->k / 256);
@@ -1518,26 +1518,15 @@ int launch_pair6(const qwen36_nvfp4_gemm_spec_t *s, float alpha) {
   return launch_pair6_form<false>(s, alpha, map_a, map_b, map_sfa, map_sfb, cfg, pairs);
 }
 
-// Split-K launch: `split` CTAs per 128-row block (cluster), one token block (n <= BN).
+template <uint32_t BN> constexpr uint32_t splitk_smem() { return Cfg<BN>::kSmemBytes + (max_split_for<BN>() - 1) * kBM * Cfg<BN>::kBRows * 4u; }
+
 template <uint32_t BN>
-int launch_splitk(const qwen36_nvfp4_gemm_spec_t *s, float alpha, uint32_t split) {
-  using C = Cfg<BN>;
-  CUtensorMap map_a, map_b;
-  if (!make_operand_map(&map_a, s->a_fp4.ptr, s->m, s->k, kBM) ||
-      !make_operand_map(&map_b, s->b_fp4.ptr, s->n, s->k, C::kBRows))
-    return QWEN36_STATUS_NOT_IMPLEMENTED;
-  constexpr uint32_t kSmem = C::kSmemBytes + (max_split_for<BN>() - 1) * kBM * C::kBRows * 4u;
-  static_assert(kSmem <= 227u * 1024u, "split-K shared memory");
-  if (split > max_split_for<BN>()) split = max_split_for<BN>();
-  if (q36::ensure_dynamic_smem(reinterpret_cast<const void *>(nvfp4_gemm_splitk_kernel<BN>), static_cast<int>(kSmem)) !=
-      cudaSuccess)
-    return QWEN36_STATUS_CUDA_ERROR;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(static_cast<uint32_t>(s->m / kBM) * split);
+void splitk_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute (&attr)[2], uint32_t m_blocks, uint32_t split) {
+  cfg = cudaLaunchConfig_t{};
+  cfg.gridDim = dim3(m_blocks * split);
   cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = kSmem;
+  cfg.dynamicSmemBytes = splitk_smem<BN>();
   cfg.stream = q36::stream();
-  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = split;
   attr[0].val.clusterDim.y = 1;
@@ -1546,22 +1535,74 @@ int launch_splitk(const qwen36_nvfp4_gemm_spec_t *s, float alpha, uint32_t split
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
+}
+
+// CTAs per row block for the split-K form (at most `most`), 1 when the plain persistent kernel should run: the one
+// that makes the longest CTA's K-blocks, over all rounds, fewest, the smaller of equals.  A cluster's CTAs share a GPC of
+// 16 to 20 SMs, so far fewer clusters fit than SMs / split: sixteen clusters of eight ran as two rounds, and so did 28 of five and
+// 36 of four.  One token, us, with SMs / row blocks as the rule | with this one: 2048 x 6144 8.2 | 4.7, 3584 x 12288 12.7 | 7.7,
+// 4608 x 16384 17.0 | 10.8; 5120 rows keep their three.
+template <uint32_t BN>
+uint32_t choose_split(const qwen36_nvfp4_gemm_spec_t *s) {
+  const uint32_t m_blocks = static_cast<uint32_t>(s->m / kBM), k_blocks = static_cast<uint32_t>(s->k / 256);
+  uint32_t most = static_cast<uint32_t>(sm_count()) / m_blocks;
+  if (const int forced = g_force_split.load(); forced > 0) most = static_cast<uint32_t>(forced);
+  if (most > max_split_for<BN>()) most = max_split_for<BN>();
+  if (most > k_blocks / 2u) most = k_blocks / 2u;                        // at least two K-blocks per CTA
+  if (most < 2u) return 1u;
+  if (g_force_split.load() > 0) return most;
+  // asked once per shape: a decode loop asks for the same few on every token
+  struct Choice { uint32_t m_blocks = 0, k_blocks = 0, split = 0, longest = 0; int dev = -1; };
+  static std::mutex mu;
+  static Choice known[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 1u;
+  Choice &slot = known[(m_blocks * 31u + k_blocks * 7u + static_cast<uint32_t>(dev)) % 64u];
+  std::lock_guard<std::mutex> lock(mu);
+  if (slot.m_blocks == m_blocks && slot.k_blocks == k_blocks && slot.dev == dev) return slot.split;
+  const void *kernel = reinterpret_cast<const void *>(nvfp4_gemm_splitk_kernel<BN>);
+  if (q36::ensure_dynamic_smem(kernel, static_cast<int>(splitk_smem<BN>())) != cudaSuccess) return 1u;
+  uint32_t best = 1u, least = k_blocks * ((m_blocks + static_cast<uint32_t>(sm_count()) - 1u) / static_cast<uint32_t>(sm_count()));
+  for (uint32_t split = 2u; split <= most; ++split) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[2];
+    splitk_config<BN>(cfg, attr, m_blocks, split);
+    const int fit = max_active_clusters(kernel, split, &cfg);
+    if (fit <= 0) continue;
+    const uint32_t rounds = (m_blocks + static_cast<uint32_t>(fit) - 1u) / static_cast<uint32_t>(fit);
+    const uint32_t longest = rounds * ((k_blocks + split - 1u) / split);
+    if (longest < least) { least = longest; best = split; }
+  }
+  slot.m_blocks = m_blocks; slot.k_blocks = k_blocks; slot.split = best; slot.longest = least; slot.dev = dev;
+  return best;
+}
+
+// Split-K launch: `split` CTAs per 128-row block (cluster), one token block (n <= BN).
+template <uint32_t BN>
+int launch_splitk(const qwen36_nvfp4_gemm_spec_t *s, float alpha, uint32_t split) {
+  using C = Cfg<BN>;
+  CUtensorMap map_a, map_b;
+  if (!make_operand_map(&map_a, s->a_fp4.ptr, s->m, s->k, kBM) ||
+      !make_operand_map(&map_b, s->b_fp4.ptr, s->n, s->k, C::kBRows))
+    return QWEN36_STATUS_NOT_IMPLEMENTED;
+  static_assert(splitk_smem<BN>() <= 227u * 1024u, "split-K shared memory");
+  if (q36::ensure_dynamic_smem(reinterpret_cast<const void *>(nvfp4_gemm_splitk_kernel<BN>), static_cast<int>(splitk_smem<BN>())) !=
+      cudaSuccess)
+    return QWEN36_STATUS_CUDA_ERROR;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr[2];
+  splitk_config<BN>(cfg, attr, static_cast<uint32_t>(s->m / kBM), split);
   return q36::cuda_status(cudaLaunchKernelEx(&cfg, nvfp4_gemm_splitk_kernel<BN>, map_a, map_b,
                                              as_ptr<const uint8_t>(s->a_scale), as_ptr<const uint8_t>(s->b_scale),
                                              as_ptr<__nv_bfloat16>(s->c_bf16), static_cast<uint32_t>(s->m),
                                              static_cast<uint32_t>(s->n), static_cast<uint32_t>(s->k), alpha));
 }
 
-// CTAs per row block for the split-K form, 1 when the plain persistent kernel should run: split
-// only when the row blocks alone leave most SMs idle, as far as that fills the device, keeping at
-// least two K-blocks per CTA.
-uint32_t choose_split(const qwen36_nvfp4_gemm_spec_t *s) {
-  const int forced = g_force_split.load();
-  const uint32_t m_blocks = static_cast<uint32_t>(s->m / kBM), k_blocks = static_cast<uint32_t>(s->k / 256);
-  uint32_t split = forced > 0 ? static_cast<uint32_t>(forced) : static_cast<uint32_t>(sm_count()) / m_blocks;
-  if (split > kMaxSplit) split = kMaxSplit;
-  if (split > k_blocks / 2u) split = k_blocks / 2u;
-  return split < 2u ? 1u : split;
+// The split-K form where it applies, the persistent kernel otherwise.
+template <uint32_t BN>
+int launch_small(const qwen36_nvfp4_gemm_spec_t *s, float alpha) {
+  const uint32_t split = choose_split<BN>(s);
+  return split > 1u ? launch_splitk<BN>(s, alpha, split) : launch<BN>(s, alpha);
 }
 
 }  // namespace
@@ -1587,23 +1628,14 @@ int nvfp4_gemm_tc(const qwen36_nvfp4_gemm_spec_t *s, float alpha) {
     const int rc = launch_pair(s, alpha);
     if (rc != QWEN36_STATUS_NOT_IMPLEMENTED) return rc;      // pairs unavailable: single-CTA tiles below
   }
-  if (s->n <= 64) {
-    // few row blocks (k / v / o / down: 8 or 40 on 148 SMs): clusters share a tile along K.  Up to 16 tokens
-    // as many CTAs per row block as fit the GPU; 32 and 64 tokens as many as the partial sums leave room for
-    // (down 5120 x 17408 at 32 tokens: 29 -> 16 us).
-    const uint32_t split = choose_split(s);
-    if (split > 1u) {
-      if (s->n <= 8) return launch_splitk<8>(s, alpha, split);
-      if (s->n <= 16) return launch_splitk<16>(s, alpha, split);
-      if (s->n <= 32) return launch_splitk<32>(s, alpha, split);
-      // two CTAs per row block: pays for long K only (k = 17408: 30 -> 23 us; k = 6144: 13.7 -> 14.6 us)
-      if (s->k >= 48u * 256u) return launch_splitk<64>(s, alpha, split);
-    }
-  }
-  if (s->n <= 8) return launch<8>(s, alpha);
-  if (s->n <= 16) return launch<16>(s, alpha);
-  if (s->n <= 32) return launch<32>(s, alpha);
-  if (s->n <= 64) return launch<64>(s, alpha);
+  // few row blocks (k / v / o / down: 8 or 40 on 148 SMs): clusters share a tile along K.  Up to 16 tokens
+  // as many CTAs per row block as fit the GPU; 32 and 64 tokens as many as the partial sums leave room for
+  // (down 5120 x 17408 at 32 tokens: 29 -> 16 us).
+  if (s->n <= 8) return launch_small<8>(s, alpha);
+  if (s->n <= 16) return launch_small<16>(s, alpha);
+  if (s->n <= 32) return launch_small<32>(s, alpha);
+  // two CTAs per row block: pays for long K only (k = 17408: 30 -> 23 us; k = 6144: 13.7 -> 14.6 us)
+  if (s->n <= 64) return s->k >= 48u * 256u ? launch_small<64>(s, alpha) : launch<64>(s, alpha);
   if (s->n <= 128) return launch<128>(s, alpha);
   return launch<256>(s, alpha);
 }

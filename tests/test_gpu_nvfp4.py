@@ -460,6 +460,18 @@ def test_w4a4_one_token_decode_vs_oracle(backend, m, k):
     assert backend.lib.qwen36_nvfp4_gemv_mma_last_error() == 0
 
 
+@pytest.mark.parametrize("m,k,n", [(2048, 1536, 5), (3584, 3072, 2), (4608, 2048, 16), (2048, 4096, 32), (1024, 3072, 8), (5120, 12288, 40)])
+def test_w4a4_split_k_with_as_many_ctas_as_have_room_together(backend, m, k, n):
+    """Row-block counts at which SMs / row blocks would give clusters that do not fit the GPU all at once (16 of eight CTAs, 28 of
+    five, 36 of four), and two that keep their split.  Only the bf16 rounding of the output (2^-9) separates it from the oracle."""
+    rng = np.random.default_rng(m + k + n)
+    a, a_sf, x, b, b_sf, alpha = w4a4_case(rng, m, n, k)
+    want = synth.bf16_bits_to_f32(orc.nvfp4_gemm(a, a_sf, b, b_sf, alpha, m, n, k))
+    got = synth.bf16_bits_to_f32(bf16_host(backend.nvfp4_gemm(to_dev(a), to_dev(a_sf), to_dev(b), to_dev(b_sf), alpha, m, n, k)))
+    assert rel_l2(got, want) <= 3e-3
+    assert backend.lib.qwen36_nvfp4_gemm_last_error() == 0
+
+
 def test_w4a4_known_answer_132_and_alpha_zero(backend):
     # kernels-cuda/smoke.cu:2140-2180
     k = m = 128
