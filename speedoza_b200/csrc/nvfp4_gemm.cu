@@ -87,7 +87,7 @@ extern "C" int qwen36_nvfp4_gemm(const qwen36_nvfp4_gemm_spec_t *spec) {
   const int rc = check(spec);
   if (rc != QWEN36_STATUS_SUCCESS) return rc;
   const float alpha = spec->alpha == 0.0f ? 1.0f : spec->alpha;   // kernels-cuda/nvfp4_gemm.cu:380
-  if (spec->n == 1 && !q36::nvfp4_gemm_tc_forced()) {              // one token: the HBM-bound GEMV
+  if (spec->n == 1 && !q36::nvfp4_gemm_tc_forced() && !q36::nvfp4_gemm_tc_for_one_token(spec)) {
     const int gv = q36::nvfp4_gemv_mma_fp4(spec, alpha);
     if (gv != QWEN36_STATUS_NOT_IMPLEMENTED) return gv;
   }
@@ -100,7 +100,7 @@ extern "C" int qwen36_decode_nvfp4_gemv(const qwen36_nvfp4_gemm_spec_t *spec) {
   const int rc = check(spec);
   if (rc != QWEN36_STATUS_SUCCESS) return rc;
   if (spec->n > 8) return QWEN36_STATUS_NOT_IMPLEMENTED;
-  if (spec->n == 1 && !q36::nvfp4_gemm_tc_forced()) {
+  if (spec->n == 1 && !q36::nvfp4_gemm_tc_forced() && !q36::nvfp4_gemm_tc_for_one_token(spec)) {
     const int gv = q36::nvfp4_gemv_mma_fp4(spec, spec->alpha);
     if (gv != QWEN36_STATUS_NOT_IMPLEMENTED) return gv;
   }

@@ -36,8 +36,9 @@
 namespace q36 {
 namespace {
 
-constexpr uint32_t kThreads = 384;            // 12 warps: 0 TMA, 1 MMA, 2 scale copier, 3 idle, 4..11 epilogue
+constexpr uint32_t kThreads = 384;            // 12 warps: 0 TMA, 1 MMA, 2 scale copier, 3 one token: scale bytes, 4..11 epilogue
 constexpr uint32_t kWarpCopier = 2;
+constexpr uint32_t kWarpScan = 3;                   // one token: looks through the scale bytes
 constexpr uint32_t kWarpEpilogue = 4;         // first epilogue warp; warp w drains TMEM lanes [32 (w % 4), +32)
 constexpr uint32_t kBM = 128;
 constexpr uint32_t kBKBytes = 128;            // 256 fp4 values
@@ -184,13 +185,46 @@ template <uint32_t BN> struct Cfg {
   static constexpr uint32_t kIdesc = (1u << 7) | (1u << 10) | ((kBRows >> 3) << 17) | ((kBM >> 4) << 24);
 };
 
+// One token: the scale bytes that the hardware reads differently.  The reference honours a scale's sign and reads 0x7F as 448; a
+// warp that has nothing else to do looks through the bytes as they land, and the rows of a tile that holds such a byte (as
+// rows whose sum is NaN) are redone with the reference's scalar arithmetic, from global memory.
+__device__ __forceinline__ uint32_t odd_scale_bytes(uint32_t w) { return w | ((w & 0x7f7f7f7fu) + 0x01010101u); }     // bit 7 of a byte: it is one
+__device__ __forceinline__ uint32_t odd_scale_bytes(const uint8_t *sfa, const uint8_t *sfb, uint32_t lane) {
+  uint32_t seen = 0u;
+#pragma unroll
+  for (uint32_t i = 0; i < 4u; ++i) {
+    const uint4 v = reinterpret_cast<const uint4 *>(sfa)[i * 32u + lane];
+    seen |= odd_scale_bytes(v.x) | odd_scale_bytes(v.y) | odd_scale_bytes(v.z) | odd_scale_bytes(v.w);
+  }
+  seen |= odd_scale_bytes(*reinterpret_cast<const uint32_t *>(sfb + (lane & 3u) * 512u));      // the token's four groups of each tile
+  return seen & 0x80808080u;
+}
+__device__ __noinline__ float exact_row(const uint8_t *w, const uint8_t *w_sf, const uint8_t *x, const uint8_t *x_sf, uint32_t row, uint32_t k,
+                                        float alpha) {
+  const uint32_t groups = k / 16u;
+  const size_t sf_inner = q36::round_up(groups, 4);
+  const uint8_t *wrow = w + static_cast<size_t>(row) * (k / 2u);
+  float sum = 0.f;
+  for (uint32_t g = 0; g < groups; ++g) {
+    float local = 0.f;
+    for (uint32_t i = 0; i < 8u; ++i) {
+      const uint32_t wb = wrow[g * 8u + i], xb = x[g * 8u + i];
+      local = fmaf(q36::e2m1_value(xb), q36::e2m1_value(wb), local);
+      local = fmaf(q36::e2m1_value(xb >> 4), q36::e2m1_value(wb >> 4), local);
+    }
+    sum = fmaf(local, __fmul_rn(q36::decode_e4m3(w_sf[q36::sf_offset(g, row, sf_inner)]), q36::decode_e4m3(x_sf[q36::sf_offset(g, 0, sf_inner)])), sum);
+  }
+  return sum * alpha;
+}
+
 // Tiles are numbered with the token block fastest: the CTAs that run at the same time cover a few
 // weight row blocks times all token blocks, so every weight tile is fetched from HBM once (its
 // other readers hit L2) and the much smaller activation matrix stays L2-resident.
-template <uint32_t BN>
+template <uint32_t BN, bool ONE>
 __global__ void __launch_bounds__(kThreads, 1)
 nvfp4_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                      const uint8_t *__restrict__ a_sf, const uint8_t *__restrict__ b_sf,
+                     const uint8_t *__restrict__ a_fp4, const uint8_t *__restrict__ b_fp4,
                      __nv_bfloat16 *__restrict__ c, uint32_t m, uint32_t n, uint32_t k, float alpha) {
   using C = Cfg<BN>;
   extern __shared__ __align__(128) uint8_t smem_raw[];
@@ -202,6 +236,8 @@ nvfp4_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   uint64_t *acc_full = sf_landed + 8;                                    // [kAccStages]
   uint64_t *acc_empty = acc_full + 2;                                    // [kAccStages]
   uint32_t *tmem_base_slot = reinterpret_cast<uint32_t *>(acc_empty + 2);
+  volatile uint32_t *scanned = reinterpret_cast<volatile uint32_t *>(smem + 512);      // one token: tiles whose scale bytes have been looked through,
+  volatile uint8_t *odd_scales = smem + 544;                                           // [32] and what was found in tile t % 32 of this CTA
   uint8_t *stages = smem + 1024;
 
   // The issuing warps (MMA, scale copier) run their loops convergent and elect a lane for the instructions alone: warp
@@ -218,9 +254,10 @@ nvfp4_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 
   if (threadIdx.x == 0) {
     for (uint32_t s = 0; s < C::kStages; ++s) {
-      mbar_init(&full[s], 1); mbar_init(&empty[s], 1); mbar_init(&sf_full[s], 1); mbar_init(&sf_landed[s], 1);
+      mbar_init(&full[s], 1); mbar_init(&empty[s], ONE ? 2 : 1); mbar_init(&sf_full[s], 1); mbar_init(&sf_landed[s], 1);
     }
     for (uint32_t s = 0; s < C::kAccStages; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], C::kEpiWarps); }
+    *scanned = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -354,6 +391,28 @@ nvfp4_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         }
       }
     }
+  } else if (ONE && warp == kWarpScan) {
+    {
+      uint32_t g = 0, t_local = 0;
+      bool dead = false;
+      for (uint32_t tile = blockIdx.x; tile < tiles && !dead; tile += gridDim.x, ++t_local) {
+        uint32_t seen = 0u;
+        for (uint32_t kb = 0; kb < k_blocks; ++kb, ++g) {
+          const uint32_t s = g % C::kStages, ph = (g / C::kStages) & 1u;
+          if (!mbar_wait_warp(&sf_landed[s], ph)) { dead = true; break; }
+          const uint8_t *sfa = stages + s * C::kStageBytes + C::kABytes + C::kBBytes;
+          seen |= odd_scale_bytes(sfa, sfa + C::kSfaBytes, lane);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&empty[s]);
+        }
+        const bool odd = __any_sync(0xffffffffu, seen != 0u);
+        if (lane == 0) {
+          odd_scales[t_local & 31u] = odd ? 1 : 0;             // the ring and the accumulators keep it far less than 32 tiles ahead
+          __threadfence_block();
+          *scanned = t_local + 1u;
+        }
+      }
+    }
   } else if (warp >= kWarpEpilogue && warp < kWarpEpilogue + C::kEpiWarps) {
     // ---------------------------------------------------------------- epilogue warps
     const uint32_t quarter = warp & 3u;           // TMEM lanes [32*quarter, +32) are this warp's
@@ -411,7 +470,13 @@ nvfp4_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 #pragma unroll
           for (uint32_t j = 0; j < 8; ++j) {
             const uint32_t tok = tok0 + c0 + j;
-            if (tok < n) c[static_cast<size_t>(tok) * m + row] = __float2bfloat16(__uint_as_float(r[j]) * alpha);
+            float v = __uint_as_float(r[j]) * alpha;
+            if (ONE && j == 0u) {
+              for (uint32_t spin = 0; *scanned <= t_local && spin < kSpinLimit; ++spin) {}    // done long ago: it waits for the scales alone
+              __threadfence_block();
+              if (odd_scales[t_local & 31u] != 0 || v != v) v = exact_row(a_fp4, a_sf, b_fp4, b_sf, row, k, alpha);
+            }
+            if (tok < n) c[static_cast<size_t>(tok) * m + row] = __float2bfloat16(v);
           }
         }
       }
@@ -1113,10 +1178,11 @@ __device__ __forceinline__ void st_cluster_v4f(uint32_t addr, float a, float b, 
   asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c4), "f"(d) : "memory");
 }
 
-template <uint32_t BN>
+template <uint32_t BN, bool ONE>
 __global__ void __launch_bounds__(kThreads, 1)
 nvfp4_gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                          const uint8_t *__restrict__ a_sf, const uint8_t *__restrict__ b_sf,
+                         const uint8_t *__restrict__ a_fp4, const uint8_t *__restrict__ b_fp4,
                          __nv_bfloat16 *__restrict__ c, uint32_t m, uint32_t n, uint32_t k, float alpha) {
   using C = Cfg<BN>;
   static_assert(BN <= 64, "split-K form is for small token counts");
@@ -1128,6 +1194,7 @@ nvfp4_gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   uint64_t *sf_full = empty + 8;
   uint64_t *acc_full = sf_full + 8;
   uint32_t *tmem_base_slot = reinterpret_cast<uint32_t *>(acc_full + 2);
+  volatile uint32_t *scanned = reinterpret_cast<volatile uint32_t *>(smem + 512);      // one token: 1 = the scale bytes have been looked through, 3 = and some are odd
   uint8_t *stages = smem + 1024;
   float *partials = reinterpret_cast<float *>(stages + C::kStages * C::kStageBytes);   // [S-1][128 rows][kCols], first CTA only
 
@@ -1143,7 +1210,8 @@ nvfp4_gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   const uint32_t sf_tiles_per_block = k / 64u;
 
   if (threadIdx.x == 0) {
-    for (uint32_t s = 0; s < C::kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); mbar_init(&sf_full[s], 1); }
+    for (uint32_t s = 0; s < C::kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], ONE ? 2 : 1); mbar_init(&sf_full[s], 1); }
+    *scanned = 0u;
     mbar_init(&acc_full[0], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -1228,6 +1296,20 @@ nvfp4_gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         __syncwarp();
       }
     }
+  } else if (ONE && warp == kWarpScan) {
+    {
+      uint32_t seen = 0u;
+      for (uint32_t kb = kb_begin, g = 0; kb < kb_end; ++kb, ++g) {
+        const uint32_t s = g % C::kStages, ph = (g / C::kStages) & 1u;
+        if (!mbar_wait_warp(&full[s], ph)) break;
+        const uint8_t *sfa = stages + s * C::kStageBytes + C::kABytes + C::kBBytes;
+        seen |= odd_scale_bytes(sfa, sfa + C::kSfaBytes, lane);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[s]);
+      }
+      const bool odd = __any_sync(0xffffffffu, seen != 0u);
+      if (lane == 0) *scanned = odd ? 3u : 1u;
+    }
   } else if (warp >= kWarpEpilogue && warp < kWarpEpilogue + 4u) {
     // epilogue warps 4..7: drain this CTA's partial sums; ranks > 0 hand them to the first CTA
     const uint32_t quarter = warp & 3u;
@@ -1245,6 +1327,11 @@ nvfp4_gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           for (uint32_t j = 0; j < 8; ++j) acc[c0 + j] = __uint_as_float(r[j]);
         }
       }
+    }
+    if (ONE) {
+      uint32_t found = *scanned;
+      for (uint32_t spin = 0; found == 0u && spin < kSpinLimit; ++spin) found = *scanned;
+      if (found != 1u) acc[0] = __uint_as_float(0x7fc00000u);            // sends the row to exact_row
     }
     if (rank != 0u) {
       const uint32_t row = quarter * 32u + lane;
@@ -1270,8 +1357,11 @@ nvfp4_gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       }
     }
 #pragma unroll
-    for (uint32_t j = 0; j < kCols; ++j)
-      if (j < n) c[static_cast<size_t>(j) * m + row] = __float2bfloat16(acc[j] * alpha);
+    for (uint32_t j = 0; j < kCols; ++j) {
+      float v = acc[j] * alpha;
+      if (ONE && j == 0u && v != v) v = exact_row(a_fp4, a_sf, b_fp4, b_sf, row, k, alpha);
+      if (j < n) c[static_cast<size_t>(j) * m + row] = __float2bfloat16(v);
+    }
   }
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -1348,22 +1438,23 @@ bool make_operand_map(CUtensorMap *map, uint64_t ptr, uint64_t rows, uint64_t k,
 
 int sm_count() { return q36::sm_count_current_device(); }
 
-template <uint32_t BN>
+template <uint32_t BN, bool ONE = false>
 int launch(const qwen36_nvfp4_gemm_spec_t *s, float alpha) {
   using C = Cfg<BN>;
   CUtensorMap map_a, map_b;
   if (!make_operand_map(&map_a, s->a_fp4.ptr, s->m, s->k, kBM) ||
       !make_operand_map(&map_b, s->b_fp4.ptr, s->n, s->k, C::kBRows))
     return QWEN36_STATUS_NOT_IMPLEMENTED;
-  if (q36::ensure_dynamic_smem(reinterpret_cast<const void *>(nvfp4_gemm_tc_kernel<BN>), static_cast<int>(C::kSmemBytes)) !=
+  if (q36::ensure_dynamic_smem(reinterpret_cast<const void *>(nvfp4_gemm_tc_kernel<BN, ONE>), static_cast<int>(C::kSmemBytes)) !=
       cudaSuccess)
     return QWEN36_STATUS_CUDA_ERROR;
   const uint32_t tiles = static_cast<uint32_t>((s->m / kBM) * ((s->n + BN - 1) / BN));
   const uint32_t grid = tiles < static_cast<uint32_t>(sm_count()) ? tiles : static_cast<uint32_t>(sm_count());
   return q36::cuda_status(q36::launch_after_previous(
-      nvfp4_gemm_tc_kernel<BN>, dim3(grid), dim3(kThreads), C::kSmemBytes, q36::stream(), map_a, map_b,
-      as_ptr<const uint8_t>(s->a_scale), as_ptr<const uint8_t>(s->b_scale), as_ptr<__nv_bfloat16>(s->c_bf16),
-      static_cast<uint32_t>(s->m), static_cast<uint32_t>(s->n), static_cast<uint32_t>(s->k), alpha));
+      nvfp4_gemm_tc_kernel<BN, ONE>, dim3(grid), dim3(kThreads), C::kSmemBytes, q36::stream(), map_a, map_b,
+      as_ptr<const uint8_t>(s->a_scale), as_ptr<const uint8_t>(s->b_scale), as_ptr<const uint8_t>(s->a_fp4),
+      as_ptr<const uint8_t>(s->b_fp4), as_ptr<__nv_bfloat16>(s->c_bf16), static_cast<uint32_t>(s->m), static_cast<uint32_t>(s->n),
+      static_cast<uint32_t>(s->k), alpha));
 }
 
 // Tiled scale buffer as uint32 [tiles][128]: one 512-byte scale tile per row, box = four tiles (one 256-K stage).
@@ -1542,13 +1633,15 @@ void splitk_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute (&attr)[2], uint
 // 16 to 20 SMs, so far fewer clusters fit than SMs / split: sixteen clusters of eight ran as two rounds, and so did 28 of five and
 // 36 of four.  One token, us, with SMs / row blocks as the rule | with this one: 2048 x 6144 8.2 | 4.7, 3584 x 12288 12.7 | 7.7,
 // 4608 x 16384 17.0 | 10.8; 5120 rows keep their three.
-template <uint32_t BN>
-uint32_t choose_split(const qwen36_nvfp4_gemm_spec_t *s) {
+template <uint32_t BN, bool ONE = false>
+uint32_t choose_split(const qwen36_nvfp4_gemm_spec_t *s, uint32_t *longest_run = nullptr) {
   const uint32_t m_blocks = static_cast<uint32_t>(s->m / kBM), k_blocks = static_cast<uint32_t>(s->k / 256);
   uint32_t most = static_cast<uint32_t>(sm_count()) / m_blocks;
   if (const int forced = g_force_split.load(); forced > 0) most = static_cast<uint32_t>(forced);
   if (most > max_split_for<BN>()) most = max_split_for<BN>();
   if (most > k_blocks / 2u) most = k_blocks / 2u;                        // at least two K-blocks per CTA
+  uint32_t best = 1u, least = k_blocks * ((m_blocks + static_cast<uint32_t>(sm_count()) - 1u) / static_cast<uint32_t>(sm_count()));
+  if (longest_run != nullptr) *longest_run = least;
   if (most < 2u) return 1u;
   if (g_force_split.load() > 0) return most;
   // asked once per shape: a decode loop asks for the same few on every token
@@ -1559,10 +1652,12 @@ uint32_t choose_split(const qwen36_nvfp4_gemm_spec_t *s) {
   if (cudaGetDevice(&dev) != cudaSuccess) return 1u;
   Choice &slot = known[(m_blocks * 31u + k_blocks * 7u + static_cast<uint32_t>(dev)) % 64u];
   std::lock_guard<std::mutex> lock(mu);
-  if (slot.m_blocks == m_blocks && slot.k_blocks == k_blocks && slot.dev == dev) return slot.split;
-  const void *kernel = reinterpret_cast<const void *>(nvfp4_gemm_splitk_kernel<BN>);
+  if (slot.m_blocks == m_blocks && slot.k_blocks == k_blocks && slot.dev == dev) {
+    if (longest_run != nullptr) *longest_run = slot.longest;
+    return slot.split;
+  }
+  const void *kernel = reinterpret_cast<const void *>(nvfp4_gemm_splitk_kernel<BN, ONE>);
   if (q36::ensure_dynamic_smem(kernel, static_cast<int>(splitk_smem<BN>())) != cudaSuccess) return 1u;
-  uint32_t best = 1u, least = k_blocks * ((m_blocks + static_cast<uint32_t>(sm_count()) - 1u) / static_cast<uint32_t>(sm_count()));
   for (uint32_t split = 2u; split <= most; ++split) {
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[2];
@@ -1573,12 +1668,13 @@ uint32_t choose_split(const qwen36_nvfp4_gemm_spec_t *s) {
     const uint32_t longest = rounds * ((k_blocks + split - 1u) / split);
     if (longest < least) { least = longest; best = split; }
   }
+  if (longest_run != nullptr) *longest_run = least;
   slot.m_blocks = m_blocks; slot.k_blocks = k_blocks; slot.split = best; slot.longest = least; slot.dev = dev;
   return best;
 }
 
 // Split-K launch: `split` CTAs per 128-row block (cluster), one token block (n <= BN).
-template <uint32_t BN>
+template <uint32_t BN, bool ONE = false>
 int launch_splitk(const qwen36_nvfp4_gemm_spec_t *s, float alpha, uint32_t split) {
   using C = Cfg<BN>;
   CUtensorMap map_a, map_b;
@@ -1586,33 +1682,52 @@ int launch_splitk(const qwen36_nvfp4_gemm_spec_t *s, float alpha, uint32_t split
       !make_operand_map(&map_b, s->b_fp4.ptr, s->n, s->k, C::kBRows))
     return QWEN36_STATUS_NOT_IMPLEMENTED;
   static_assert(splitk_smem<BN>() <= 227u * 1024u, "split-K shared memory");
-  if (q36::ensure_dynamic_smem(reinterpret_cast<const void *>(nvfp4_gemm_splitk_kernel<BN>), static_cast<int>(splitk_smem<BN>())) !=
+  if (q36::ensure_dynamic_smem(reinterpret_cast<const void *>(nvfp4_gemm_splitk_kernel<BN, ONE>), static_cast<int>(splitk_smem<BN>())) !=
       cudaSuccess)
     return QWEN36_STATUS_CUDA_ERROR;
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[2];
   splitk_config<BN>(cfg, attr, static_cast<uint32_t>(s->m / kBM), split);
-  return q36::cuda_status(cudaLaunchKernelEx(&cfg, nvfp4_gemm_splitk_kernel<BN>, map_a, map_b,
+  return q36::cuda_status(cudaLaunchKernelEx(&cfg, nvfp4_gemm_splitk_kernel<BN, ONE>, map_a, map_b,
                                              as_ptr<const uint8_t>(s->a_scale), as_ptr<const uint8_t>(s->b_scale),
+                                             as_ptr<const uint8_t>(s->a_fp4), as_ptr<const uint8_t>(s->b_fp4),
                                              as_ptr<__nv_bfloat16>(s->c_bf16), static_cast<uint32_t>(s->m),
                                              static_cast<uint32_t>(s->n), static_cast<uint32_t>(s->k), alpha));
 }
 
 // The split-K form where it applies, the persistent kernel otherwise.
-template <uint32_t BN>
+template <uint32_t BN, bool ONE = false>
 int launch_small(const qwen36_nvfp4_gemm_spec_t *s, float alpha) {
-  const uint32_t split = choose_split<BN>(s);
-  return split > 1u ? launch_splitk<BN>(s, alpha, split) : launch<BN>(s, alpha);
+  const uint32_t split = choose_split<BN, ONE>(s);
+  return split > 1u ? launch_splitk<BN, ONE>(s, alpha, split) : launch<BN, ONE>(s, alpha);
+}
+
+bool operands_fit(const qwen36_nvfp4_gemm_spec_t *s) {
+  return s->m % kBM == 0 && s->k % 256 == 0 && s->m <= (1u << 30) && s->n <= (1u << 30) && s->k <= (1u << 30) &&
+         ((s->a_fp4.ptr | s->b_fp4.ptr | s->a_scale.ptr | s->b_scale.ptr) & 15u) == 0 && (s->c_bf16.ptr & 3u) == 0;
 }
 
 }  // namespace
 
 bool nvfp4_gemm_tc_forced() { return g_force_bn.load() != 0 || g_force_split.load() != 0; }
 
+// One token: this kernel where its CTAs are evenly busy, at least 0.62 of the SMs' K-blocks at the rate of the longest run; else the
+// GEMV, whose units are smaller.  us a launch behind a small producer, GEMV | this one, and that share: 34816 x 5120 23.9 | 20.0 (0.92),
+// 5120 x 17408 16.1 | 13.1 (0.80), 12288 x 5120 13.0 | 11.0 (0.65), 24576 x 3584 14.4 | 13.8 (0.65), 12288 x 2048 8.0 | 7.2 (0.65),
+// 22016 x 5120 17.3 | 18.2 (0.58).  At full HBM rate the GEMV's conversions leave an SM hardly faster than its share of HBM, so that it
+// cannot work off what was prefetched while the producer ran.  Eight feed-forward blocks of 5120 x 17408, norm and SwiGLU included:
+// 319.4 -> 278.9 us; 3584 x 12288 210.5 -> 202.3, 2048 x 6144 125.7 -> 127.0.  A kernel of its own (ONE): the scan of the scale bytes in
+// the kernel for two to eight tokens made those 1.2 % slower.
+bool nvfp4_gemm_tc_for_one_token(const qwen36_nvfp4_gemm_spec_t *s) {
+  if (!operands_fit(s) || s->n != 1) return false;
+  uint32_t longest = 0;
+  choose_split<8, true>(s, &longest);
+  const uint64_t work = static_cast<uint64_t>(s->m / kBM) * (s->k / 256), room = static_cast<uint64_t>(sm_count()) * longest;
+  return work * 100u >= room * 62u;
+}
+
 int nvfp4_gemm_tc(const qwen36_nvfp4_gemm_spec_t *s, float alpha) {
-  if (s->m % kBM != 0 || s->k % 256 != 0 || s->m > (1u << 30) || s->n > (1u << 30) || s->k > (1u << 30) ||
-      ((s->a_fp4.ptr | s->b_fp4.ptr | s->a_scale.ptr | s->b_scale.ptr) & 15u) != 0 || (s->c_bf16.ptr & 3u) != 0)
-    return QWEN36_STATUS_NOT_IMPLEMENTED;
+  if (!operands_fit(s)) return QWEN36_STATUS_NOT_IMPLEMENTED;
   const int forced = g_force_bn.load();
   if (forced == 128 && s->n > 128) return launch<128>(s, alpha);
   // CTA pairs (256 x 256 tiles): measured ahead of single-CTA tiles only for long K with many
@@ -1631,6 +1746,7 @@ int nvfp4_gemm_tc(const qwen36_nvfp4_gemm_spec_t *s, float alpha) {
   // few row blocks (k / v / o / down: 8 or 40 on 148 SMs): clusters share a tile along K.  Up to 16 tokens
   // as many CTAs per row block as fit the GPU; 32 and 64 tokens as many as the partial sums leave room for
   // (down 5120 x 17408 at 32 tokens: 29 -> 16 us).
+  if (s->n == 1) return launch_small<8, true>(s, alpha);
   if (s->n <= 8) return launch_small<8>(s, alpha);
   if (s->n <= 16) return launch_small<16>(s, alpha);
   if (s->n <= 32) return launch_small<32>(s, alpha);

@@ -472,6 +472,30 @@ def test_w4a4_split_k_with_as_many_ctas_as_have_room_together(backend, m, k, n):
     assert backend.lib.qwen36_nvfp4_gemm_last_error() == 0
 
 
+@pytest.mark.parametrize("m,k", [(12288, 256), (5120, 1536), (37632, 512), (11904, 256)])
+def test_w4a4_one_token_every_scale_byte(backend, m, k):
+    """One token where the block-scaled MMA takes it (one tile a CTA, clusters along K, two rounds) and where the GEMV does: all
+    256 scale bytes among the weights of some row blocks, whose signs and 0x7F the reference honours, ordinary ones elsewhere."""
+    rng = np.random.default_rng(m + k)
+    packed = rng.integers(0, 256, size=(m, k // 2), dtype=np.uint8)
+    sf_rm = rng.integers(synth.SF_CODE_LO, synth.SF_CODE_HI + 1, size=(m, k // 16), dtype=np.uint8)
+    odd = rng.choice(m // 128, 6, replace=False)
+    for i, blk in enumerate(odd):                      # whole blocks, single rows, a single byte
+        rows = slice(blk * 128, blk * 128 + 128) if i < 2 else blk * 128 + rng.integers(0, 128, 3)
+        sf_rm[rows] = rng.integers(0, 256, size=sf_rm[rows].shape, dtype=np.uint8)
+    sf_rm[odd[0] * 128 + 127, -1] = 0x7F
+    sf_rm[odd[5] * 128, 0] = 0xC0
+    a_sf = orc.retile_scales(sf_rm)
+    b, b_sf, ts = orc.nvfp4_quantize_rows(synth.activations(rng, 1, k), 0.4)
+    alpha = 0.01 * ts
+    want = synth.bf16_bits_to_f32(orc.nvfp4_gemm(packed, a_sf, b, b_sf, alpha, m, 1, k))
+    got = synth.bf16_bits_to_f32(bf16_host(backend.nvfp4_gemm(to_dev(packed), to_dev(a_sf), to_dev(b), to_dev(b_sf), alpha, m, 1, k)))
+    assert np.isfinite(got).all() and rel_l2(got, want) <= 3e-3
+    plain = np.setdiff1d(np.arange(m), (odd[:, None] * 128 + np.arange(128)).ravel())
+    assert rel_l2(got[:, plain], want[:, plain]) <= 3e-3
+    assert backend.lib.qwen36_nvfp4_gemm_last_error() == 0
+
+
 def test_w4a4_known_answer_132_and_alpha_zero(backend):
     # kernels-cuda/smoke.cu:2140-2180
     k = m = 128
