@@ -465,6 +465,17 @@ decode_split_fp8_staged_kernel(const __nv_bfloat16 *__restrict__ q, const uint8_
   const uint32_t head0 = blockIdx.x * G;
   const uint32_t kvh = head0 / q_per_kv;
   const uint32_t split = blockIdx.y;
+  if (position_device == nullptr && n_splits >= q36::kAheadFrom) {
+    // meanwhile L2 is asked for the split's first tokens, contiguous over the kv heads: every CTA of the split takes an equal part
+    size_t from, to;
+    split_range(position_scalar, n_splits, split, from, to);
+    const size_t ahead = min(to - from, static_cast<size_t>(q36::kSplitAhead));
+    const size_t first = from + ahead * blockIdx.x / gridDim.x, last = from + ahead * (blockIdx.x + 1u) / gridDim.x;
+    const size_t pitch = static_cast<size_t>(kv_heads) * 256;
+    const uint32_t bytes = static_cast<uint32_t>((last - first) * pitch);
+    q36::prefetch_l2_span(reinterpret_cast<const uint8_t *>(cache_k) + first * pitch, bytes, threadIdx.x);
+    q36::prefetch_l2_span(reinterpret_cast<const uint8_t *>(cache_v) + first * pitch, bytes, kThreads - 1u - threadIdx.x);
+  }
   asm volatile("griddepcontrol.wait;" ::: "memory");       // seated early; nothing is touched before the previous kernel is done
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const size_t position = read_position(position_scalar, position_device);
@@ -559,6 +570,17 @@ decode_split_bf16_mma_kernel(const __nv_bfloat16 *__restrict__ q, const __nv_bfl
   const uint32_t head0 = blockIdx.x * G;
   const uint32_t kvh = head0 / q_per_kv;
   const uint32_t split = blockIdx.y;
+  if (position_device == nullptr && n_splits >= q36::kAheadFrom) {
+    // meanwhile L2 is asked for the split's first tokens, contiguous over the kv heads: every CTA of the split takes an equal part
+    size_t from, to;
+    split_range(position_scalar, n_splits, split, from, to);
+    const size_t ahead = min(to - from, static_cast<size_t>(q36::kSplitAhead));
+    const size_t first = from + ahead * blockIdx.x / gridDim.x, last = from + ahead * (blockIdx.x + 1u) / gridDim.x;
+    const size_t pitch = static_cast<size_t>(kv_heads) * 512;
+    const uint32_t bytes = static_cast<uint32_t>((last - first) * pitch);
+    q36::prefetch_l2_span(reinterpret_cast<const uint8_t *>(cache_k) + first * pitch, bytes, threadIdx.x);
+    q36::prefetch_l2_span(reinterpret_cast<const uint8_t *>(cache_v) + first * pitch, bytes, kThreads - 1u - threadIdx.x);
+  }
   asm volatile("griddepcontrol.wait;" ::: "memory");       // seated early; nothing is touched before the previous kernel is done
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const size_t position = read_position(position_scalar, position_device);

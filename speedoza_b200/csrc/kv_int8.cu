@@ -925,6 +925,15 @@ kv_attention_staged_kernel(const __nv_bfloat16 *__restrict__ q, const int8_t *__
   const uint32_t cta_flat = blockIdx.y * gridDim.x + blockIdx.x;
   (void)cta_flat;
   Q36_ATRACE(cta_flat, 0);
+  if (n_splits >= q36::kAheadFrom) {
+    // Meanwhile L2 is asked for the split's first kSplitAhead tokens, which lie contiguous over the kv heads: every CTA of the split
+    // takes an equal part.
+    const size_t ahead = min(s_end - s_begin, static_cast<size_t>(q36::kSplitAhead));
+    const size_t first = s_begin + ahead * blockIdx.x / gridDim.x, last = s_begin + ahead * (blockIdx.x + 1u) / gridDim.x;
+    const uint32_t bytes = static_cast<uint32_t>((last - first) * kv_heads * D);
+    q36::prefetch_l2_span(reinterpret_cast<const uint8_t *>(kq) + first * kv_heads * D, bytes, threadIdx.x);
+    q36::prefetch_l2_span(reinterpret_cast<const uint8_t *>(vq) + first * kv_heads * D, bytes, kThreads - 1u - threadIdx.x);
+  }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   Q36_ATRACE(cta_flat, 1);
