@@ -237,8 +237,8 @@ class CudaBackend:
         rows, vocab = logits_bf16.shape
         cols = weight_bf16.shape[1]
         dev = logits_bf16.device
-        tokens = torch.zeros(rows, dtype=torch.int32, device=dev)
-        flags = torch.zeros(rows, dtype=torch.int32, device=dev)
+        tokens = torch.empty(rows, dtype=torch.int32, device=dev)   # every row of both is written
+        flags = torch.empty(rows, dtype=torch.int32, device=dev)
         ws = torch.empty(rows * self.TOP2_BLOCKS * 16, dtype=torch.uint8, device=dev)
         spec = abi.LmHeadTop8RescoreSpec(rows, vocab, cols, eps, _dp(logits_bf16), _dp(weight_bf16), _dp(input_bf16),
                                          _dp(tokens), _dp(flags), _dp(mirror), _dp(fallback_count), _dp(ws), ws.numel())
