@@ -99,6 +99,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
   atomicExch(&g_gemm_error, 1u);
   return false;
 }
+// A count in shared memory that another warp of the CTA raises to `want`.
+__device__ __forceinline__ bool count_wait(const volatile uint32_t *count, uint32_t want) {
+  for (uint32_t spin = 0; spin < kSpinLimit; ++spin)
+    if (*count >= want) {
+      __threadfence_block();
+      return true;
+    }
+  atomicExch(&g_gemm_error, 1u);
+  return false;
+}
 // For a whole warp: the verdict is the same in every lane, so that the code behind it stays convergent.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity));
@@ -472,9 +482,9 @@ nvfp4_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             const uint32_t tok = tok0 + c0 + j;
             float v = __uint_as_float(r[j]) * alpha;
             if (ONE && j == 0u) {
-              for (uint32_t spin = 0; *scanned <= t_local && spin < kSpinLimit; ++spin) {}    // done long ago: it waits for the scales alone
-              __threadfence_block();
-              if (odd_scales[t_local & 31u] != 0 || v != v) v = exact_row(a_fp4, a_sf, b_fp4, b_sf, row, k, alpha);
+              // done long ago: it waits for the scales alone; a tile without a verdict counts as odd
+              if (!count_wait(scanned, t_local + 1u) || odd_scales[t_local & 31u] != 0 || v != v)
+                v = exact_row(a_fp4, a_sf, b_fp4, b_sf, row, k, alpha);
             }
             if (tok < n) c[static_cast<size_t>(tok) * m + row] = __float2bfloat16(v);
           }
@@ -1328,11 +1338,7 @@ nvfp4_gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         }
       }
     }
-    if (ONE) {
-      uint32_t found = *scanned;
-      for (uint32_t spin = 0; found == 0u && spin < kSpinLimit; ++spin) found = *scanned;
-      if (found != 1u) acc[0] = __uint_as_float(0x7fc00000u);            // sends the row to exact_row
-    }
+    if (ONE && (!count_wait(scanned, 1u) || *scanned != 1u)) acc[0] = __uint_as_float(0x7fc00000u);   // sends the row to exact_row
     if (rank != 0u) {
       const uint32_t row = quarter * 32u + lane;
       const uint32_t dst = map_to_cta(smem_u32(partials + (static_cast<size_t>(rank - 1u) * kBM + row) * kCols), 0u);
