@@ -1717,19 +1717,39 @@ bool operands_fit(const qwen36_nvfp4_gemm_spec_t *s) {
 
 bool nvfp4_gemm_tc_forced() { return g_force_bn.load() != 0 || g_force_split.load() != 0; }
 
-// One token: this kernel where its CTAs are evenly busy, at least 0.62 of the SMs' K-blocks at the rate of the longest run; else the
-// GEMV, whose units are smaller.  us a launch behind a small producer, GEMV | this one, and that share: 34816 x 5120 23.9 | 20.0 (0.92),
-// 5120 x 17408 16.1 | 13.1 (0.80), 12288 x 5120 13.0 | 11.0 (0.65), 24576 x 3584 14.4 | 13.8 (0.65), 12288 x 2048 8.0 | 7.2 (0.65),
-// 22016 x 5120 17.3 | 18.2 (0.58).  At full HBM rate the GEMV's conversions leave an SM hardly faster than its share of HBM, so that it
-// cannot work off what was prefetched while the producer ran.  Eight feed-forward blocks of 5120 x 17408, norm and SwiGLU included:
-// 319.4 -> 278.9 us; 3584 x 12288 210.5 -> 202.3, 2048 x 6144 125.7 -> 127.0.  A kernel of its own (ONE): the scan of the scale bytes in
-// the kernel for two to eight tokens made those 1.2 % slower.
+// One token: this kernel where it is the faster one, ahead of the GEMV, whose units (32 rows) are smaller and whose weights are on their
+// way before it waits.  At full HBM rate the GEMV's conversions leave an SM hardly faster than its share of HBM, so that it cannot
+// work off what was prefetched while the producer ran.  What decides is the share of the SMs that is busy: K-blocks over what the SMs
+// could do in the longest run.  About five hundred shapes were timed, replayed over cold weights, behind the row quantiser, the norm
+// and SwiGLU, and 208 feed-forward blocks (eight in a row).  GEMV | this one, us a launch behind each of the three:
+//  * Tiles, one per CTA: from 0.62 (12288 x 5120 13.0 11.2, 13.3 12.6, 12.7 10.9; 18944 x 4096 12.6 11.4, 12.9 12.6, 12.1 11.2); short K from
+//    0.70 (12288 x 2048, 0.65: 8.1 7.2, but 8.4 8.5 and 6.9 7.1).  The GEMV goes through K in steps of 1024, so other K count as the next
+//    multiple: eight blocks of 2304 x 6144 take 129.8 us with tiles for gate_up, 135.7 with the GEMV; of 2048 x 6144 126.5 and 123.6.
+//  * More rounds of tiles (the GEMV has none): from 0.72 for two (28672 x 5120 20.8 18.7, 21.9 20.1, 20.8 18.5; 24576 x 4096, 0.65: 15.3
+//    15.9, 15.8 17.0, 15.8 15.4), 0.78 for more (44800 x 5120, 0.79: 28.6 26.7, 29.5 28.5, 28.2 26.5; 57344 x 4096, 0.76: 27.2 28.4); shorter
+//    K sooner, from 0.69 below 4096 and 0.62 below 3072 (eight blocks: 3072 x 11776, 0.62, 184.6 us with the GEMV for gate_up, 187.6 with
+//    tiles; 3584 x 11264, 0.68, 196.3 199.9; 3072 x 13824, 0.73, 203.5 190.7; 2048 x 11776, 0.62, 165.4 161.5).
+//  * Clusters: from 0.60 (2048 x 17408, 0.61: 11.8 9.3).  They cost 0.6 us more than one CTA per tile, so K has to be long: from 3584
+//    where every SM has more than one of the GEMV's units (5632 x 3584 7.3 6.8, 8.3 7.7, 7.1 6.9; x 2048 5.5 5.8), from 6144 where it has
+//    one at most (3072 x 6656 8.5 7.1, 9.9 8.6, 8.6 7.1; x 6144 7.0 6.9, 8.5 8.4, 6.7 7.0; x 5120 6.3 6.6, 7.9 7.9, 6.2 6.6), above 8192 where
+//    that leaves most SMs free (1536 x 8192 6.5 6.9, 8.3 8.8, 6.5 6.8).
+// A kernel of its own (ONE): the scan of the scale bytes in the kernel for two to eight tokens made those 1.2 % slower.
 bool nvfp4_gemm_tc_for_one_token(const qwen36_nvfp4_gemm_spec_t *s) {
   if (!operands_fit(s) || s->n != 1) return false;
   uint32_t longest = 0;
-  choose_split<8, true>(s, &longest);
-  const uint64_t work = static_cast<uint64_t>(s->m / kBM) * (s->k / 256), room = static_cast<uint64_t>(sm_count()) * longest;
-  return work * 100u >= room * 62u;
+  const uint32_t split = choose_split<8, true>(s, &longest);
+  const uint32_t sms = static_cast<uint32_t>(sm_count()), k = static_cast<uint32_t>(s->k);
+  const uint32_t m_blocks = static_cast<uint32_t>(s->m / kBM), rounds = (m_blocks + sms - 1u) / sms;
+  uint32_t k_blocks = k / 256u, least;                                   // least share, percent
+  if (split > 1u) {
+    const uint32_t units = 4u * m_blocks;                                // the GEMV's
+    if (k < (units > sms ? 3584u : units * 5u > sms * 2u ? 6144u : 8448u)) return false;
+    least = 60u;
+  } else {
+    k_blocks = static_cast<uint32_t>(q36::round_up(k_blocks, 4));
+    least = rounds == 1u ? (k < 3072u ? 70u : 62u) : k < 3072u ? 62u : k < 4096u ? 69u : rounds == 2u ? 72u : 78u;
+  }
+  return static_cast<uint64_t>(m_blocks) * k_blocks * 100u >= static_cast<uint64_t>(sms) * longest * least;
 }
 
 int nvfp4_gemm_tc(const qwen36_nvfp4_gemm_spec_t *s, float alpha) {
