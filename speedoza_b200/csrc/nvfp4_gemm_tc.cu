@@ -99,16 +99,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
   atomicExch(&g_gemm_error, 1u);
   return false;
 }
-// A count in shared memory that another warp of the CTA raises to `want`.
-__device__ __forceinline__ bool count_wait(const volatile uint32_t *count, uint32_t want) {
-  for (uint32_t spin = 0; spin < kSpinLimit; ++spin)
-    if (*count >= want) {
-      __threadfence_block();
-      return true;
-    }
-  atomicExch(&g_gemm_error, 1u);
-  return false;
-}
 // For a whole warp: the verdict is the same in every lane, so that the code behind it stays convergent.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity));
@@ -195,36 +185,90 @@ template <uint32_t BN> struct Cfg {
   static constexpr uint32_t kIdesc = (1u << 7) | (1u << 10) | ((kBRows >> 3) << 17) | ((kBM >> 4) << 24);
 };
 
-// One token: the scale bytes that the hardware reads differently.  The reference honours a scale's sign and reads 0x7F as 448; a
-// warp that has nothing else to do looks through the bytes as they land, and the rows of a tile that holds such a byte (as
-// rows whose sum is NaN) are redone with the reference's scalar arithmetic, from global memory.
-__device__ __forceinline__ uint32_t odd_scale_bytes(uint32_t w) { return w | ((w & 0x7f7f7f7fu) + 0x01010101u); }     // bit 7 of a byte: it is one
-__device__ __forceinline__ uint32_t odd_scale_bytes(const uint8_t *sfa, const uint8_t *sfb, uint32_t lane) {
-  uint32_t seen = 0u;
+// One token: the scale bytes that the hardware reads differently.  The reference honours a scale's sign and reads 0x7F as 448.  A
+// warp that has nothing else to do looks through the bytes as they land (0x80 is zero on both sides) and notes the rows that hold such
+// a byte, or all of them where the token does; when the tiles are stored, all warps redo the noted rows from global memory.  The
+// roles that store wait for nothing and test nothing.  MEASURED_HERE
+__device__ __forceinline__ uint32_t odd_scale_bytes(uint32_t w) {                       // bit 7 of a byte: it is one
+  const uint32_t size = w & 0x7f7f7f7fu;
+  return (w & (size + 0x7f7f7f7fu)) | (size + 0x01010101u);
+}
+// A stage: four words of each scale tile at 16 lane are the four groups of rows lane, 32 + lane, 64 + lane and 96 + lane, and the
+// first word of a token's tile its four groups.  The stage goes back to the ring behind this warp, so two operations a word look first
+// whether there can be any (an overflow into the next byte comes from one that counts itself).
+__device__ __forceinline__ void scan_scale_bytes(const uint8_t *sfa, const uint8_t *sfb, uint32_t lane, uint32_t (&rows)[4], uint32_t &token) {
+  uint4 v[4];
+#pragma unroll
+  for (uint32_t i = 0; i < 4u; ++i) v[i] = reinterpret_cast<const uint4 *>(sfa)[i * 32u + lane];
+  const uint32_t t = *reinterpret_cast<const uint32_t *>(sfb + (lane & 3u) * 512u);
+  uint32_t seen = t | (t + 0x01010101u);
 #pragma unroll
   for (uint32_t i = 0; i < 4u; ++i) {
-    const uint4 v = reinterpret_cast<const uint4 *>(sfa)[i * 32u + lane];
-    seen |= odd_scale_bytes(v.x) | odd_scale_bytes(v.y) | odd_scale_bytes(v.z) | odd_scale_bytes(v.w);
+    seen |= v[i].x | (v[i].x + 0x01010101u); seen |= v[i].y | (v[i].y + 0x01010101u);
+    seen |= v[i].z | (v[i].z + 0x01010101u); seen |= v[i].w | (v[i].w + 0x01010101u);
   }
-  seen |= odd_scale_bytes(*reinterpret_cast<const uint32_t *>(sfb + (lane & 3u) * 512u));      // the token's four groups of each tile
-  return seen & 0x80808080u;
+  if ((seen & 0x80808080u) == 0u) return;
+#pragma unroll
+  for (uint32_t i = 0; i < 4u; ++i) {
+    rows[0] |= odd_scale_bytes(v[i].x); rows[1] |= odd_scale_bytes(v[i].y); rows[2] |= odd_scale_bytes(v[i].z); rows[3] |= odd_scale_bytes(v[i].w);
+  }
+  token |= odd_scale_bytes(t);
 }
-__device__ __noinline__ float exact_row(const uint8_t *w, const uint8_t *w_sf, const uint8_t *x, const uint8_t *x_sf, uint32_t row, uint32_t k,
-                                        float alpha) {
-  const uint32_t groups = k / 16u;
-  const size_t sf_inner = q36::round_up(groups, 4);
-  const uint8_t *wrow = w + static_cast<size_t>(row) * (k / 2u);
-  float sum = 0.f;
-  for (uint32_t g = 0; g < groups; ++g) {
-    float local = 0.f;
-    for (uint32_t i = 0; i < 8u; ++i) {
-      const uint32_t wb = wrow[g * 8u + i], xb = x[g * 8u + i];
-      local = fmaf(q36::e2m1_value(xb), q36::e2m1_value(wb), local);
-      local = fmaf(q36::e2m1_value(xb >> 4), q36::e2m1_value(wb >> 4), local);
-    }
-    sum = fmaf(local, __fmul_rn(q36::decode_e4m3(w_sf[q36::sf_offset(g, row, sf_inner)]), q36::decode_e4m3(x_sf[q36::sf_offset(g, 0, sf_inner)])), sum);
+// A whole warp, once per tile: bit r of word q says that row 32 q + r is to be redone.
+__device__ __forceinline__ uint4 odd_rows_of(const uint32_t (&rows)[4], uint32_t token) {
+  if (!__any_sync(0xffffffffu, ((rows[0] | rows[1] | rows[2] | rows[3] | token) & 0x80808080u) != 0u)) return make_uint4(0u, 0u, 0u, 0u);
+  const bool all = __any_sync(0xffffffffu, (token & 0x80808080u) != 0u);
+  uint32_t found[4];
+#pragma unroll
+  for (uint32_t q = 0; q < 4u; ++q) found[q] = __ballot_sync(0xffffffffu, all || (rows[q] & 0x80808080u) != 0u);
+  return make_uint4(found[0], found[1], found[2], found[3]);
+}
+// Eight products of E2M1 codes, times four: twice the magnitudes by table, the signs as a complement on one side.
+__device__ __forceinline__ int e2m1_dot8_x4(uint32_t w, uint32_t x, int sum) {
+  const uint32_t sign = ((w ^ x) >> 3) & 0x11111111u;
+#pragma unroll
+  for (uint32_t half = 0; half < 32u; half += 16u) {
+    const uint32_t wm = __byte_perm(0x03020100u, 0x0c080604u, (w >> half) & 0x7777u), xm = __byte_perm(0x03020100u, 0x0c080604u, (x >> half) & 0x7777u);
+    const uint32_t minus = __byte_perm(0x0000ff00u, 0u, (sign >> half) & 0x1111u);
+    sum = __dp4a(static_cast<int>(wm ^ minus), static_cast<int>(xm), sum);            // -v = ~v + 1
+    sum = __dp4a(static_cast<int>(minus & 0x01010101u), static_cast<int>(xm), sum);
   }
-  return sum * alpha;
+  return sum;
+}
+// A whole CTA: the rows row0 + 32 q + r of the bits r of noted[q], a warp each.  Latency bounds a row, so 64 pairs of groups are on
+// their way at a time.
+__device__ __noinline__ void redo_rows(const uint32_t *noted, const uint8_t *w, const uint8_t *w_sf, const uint8_t *x, const uint8_t *x_sf,
+                                       __nv_bfloat16 *c, uint32_t row0, uint32_t k, float alpha) {
+  constexpr uint32_t kBatch = 2;
+  const uint32_t lane = threadIdx.x & 31u, pairs = k / 32u;
+  for (uint32_t in = threadIdx.x >> 5; in < kBM; in += kThreads / 32u) {
+    if (((noted[in >> 5] >> (in & 31u)) & 1u) == 0u) continue;
+    const uint32_t row = row0 + in;
+    const uint4 *wrow = reinterpret_cast<const uint4 *>(w + static_cast<size_t>(row) * (k / 2u)), *xrow = reinterpret_cast<const uint4 *>(x);
+    const uint8_t *wsf = w_sf + q36::sf_offset(0, row, k / 16u);
+    float sum = 0.f;
+    for (uint32_t p0 = lane; p0 < pairs; p0 += 32u * kBatch) {
+      uint4 wv[kBatch], xv[kBatch];
+      uint32_t ws[kBatch], xs[kBatch];
+#pragma unroll
+      for (uint32_t i = 0; i < kBatch; ++i) {                                         // past the end: the first pair, with scales of zero
+        const uint32_t p = p0 + 32u * i < pairs ? p0 + 32u * i : 0u, at = (p / 2u) * 512u + (p % 2u) * 2u;
+        wv[i] = wrow[p]; xv[i] = xrow[p];
+        ws[i] = *reinterpret_cast<const uint16_t *>(wsf + at); xs[i] = *reinterpret_cast<const uint16_t *>(x_sf + at);
+        if (p0 + 32u * i >= pairs) ws[i] = 0u;
+      }
+#pragma unroll
+      for (uint32_t i = 0; i < kBatch; ++i) {                                         // a group's sum is exact
+        const int lo = e2m1_dot8_x4(wv[i].y, xv[i].y, e2m1_dot8_x4(wv[i].x, xv[i].x, 0));
+        const int hi = e2m1_dot8_x4(wv[i].w, xv[i].w, e2m1_dot8_x4(wv[i].z, xv[i].z, 0));
+        sum = fmaf(0.25f * static_cast<float>(lo), __fmul_rn(q36::decode_e4m3(ws[i] & 0xffu), q36::decode_e4m3(xs[i] & 0xffu)), sum);
+        sum = fmaf(0.25f * static_cast<float>(hi), __fmul_rn(q36::decode_e4m3(ws[i] >> 8), q36::decode_e4m3(xs[i] >> 8)), sum);
+      }
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    if (lane == 0) c[row] = __float2bfloat16(sum * alpha);
+  }
 }
 
 // Tiles are numbered with the token block fastest: the CTAs that run at the same time cover a few
@@ -246,8 +290,8 @@ nvfp4_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   uint64_t *acc_full = sf_landed + 8;                                    // [kAccStages]
   uint64_t *acc_empty = acc_full + 2;                                    // [kAccStages]
   uint32_t *tmem_base_slot = reinterpret_cast<uint32_t *>(acc_empty + 2);
-  volatile uint32_t *scanned = reinterpret_cast<volatile uint32_t *>(smem + 512);      // one token: tiles whose scale bytes have been looked through,
-  volatile uint8_t *odd_scales = smem + 544;                                           // [32] and what was found in tile t % 32 of this CTA
+  uint32_t *any_odd = reinterpret_cast<uint32_t *>(smem + 384);          // one token: are there rows to redo,
+  uint4 *odd_rows = reinterpret_cast<uint4 *>(smem + 512);               // [32] and which, of the tiles t, t + 32, .. of this CTA together
   uint8_t *stages = smem + 1024;
 
   // The issuing warps (MMA, scale copier) run their loops convergent and elect a lane for the instructions alone: warp
@@ -267,7 +311,6 @@ nvfp4_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
       mbar_init(&full[s], 1); mbar_init(&empty[s], ONE ? 2 : 1); mbar_init(&sf_full[s], 1); mbar_init(&sf_landed[s], 1);
     }
     for (uint32_t s = 0; s < C::kAccStages; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], C::kEpiWarps); }
-    *scanned = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -403,25 +446,29 @@ nvfp4_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     }
   } else if (ONE && warp == kWarpScan) {
     {
-      uint32_t g = 0, t_local = 0;
+      uint32_t g = 0, t_local = 0, any = 0u;
       bool dead = false;
       for (uint32_t tile = blockIdx.x; tile < tiles && !dead; tile += gridDim.x, ++t_local) {
-        uint32_t seen = 0u;
+        uint32_t rows[4] = {0u, 0u, 0u, 0u}, token = 0u;
         for (uint32_t kb = 0; kb < k_blocks; ++kb, ++g) {
           const uint32_t s = g % C::kStages, ph = (g / C::kStages) & 1u;
           if (!mbar_wait_warp(&sf_landed[s], ph)) { dead = true; break; }
           const uint8_t *sfa = stages + s * C::kStageBytes + C::kABytes + C::kBBytes;
-          seen |= odd_scale_bytes(sfa, sfa + C::kSfaBytes, lane);
+          scan_scale_bytes(sfa, sfa + C::kSfaBytes, lane, rows, token);
           __syncwarp();
           if (lane == 0) mbar_arrive(&empty[s]);
         }
-        const bool odd = __any_sync(0xffffffffu, seen != 0u);
+        uint4 found = odd_rows_of(rows, token);
+        any |= found.x | found.y | found.z | found.w;
         if (lane == 0) {
-          odd_scales[t_local & 31u] = odd ? 1 : 0;             // the ring and the accumulators keep it far less than 32 tiles ahead
-          __threadfence_block();
-          *scanned = t_local + 1u;
+          if (t_local >= 32u) {
+            const uint4 with = odd_rows[t_local & 31u];
+            found.x |= with.x; found.y |= with.y; found.z |= with.z; found.w |= with.w;
+          }
+          odd_rows[t_local & 31u] = found;
         }
       }
+      if (lane == 0) *any_odd = dead ? 0u : any;               // a wait that ran out has been recorded
     }
   } else if (warp >= kWarpEpilogue && warp < kWarpEpilogue + C::kEpiWarps) {
     // ---------------------------------------------------------------- epilogue warps
@@ -480,13 +527,7 @@ nvfp4_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 #pragma unroll
           for (uint32_t j = 0; j < 8; ++j) {
             const uint32_t tok = tok0 + c0 + j;
-            float v = __uint_as_float(r[j]) * alpha;
-            if (ONE && j == 0u) {
-              // done long ago: it waits for the scales alone; a tile without a verdict counts as odd
-              if (!count_wait(scanned, t_local + 1u) || odd_scales[t_local & 31u] != 0 || v != v)
-                v = exact_row(a_fp4, a_sf, b_fp4, b_sf, row, k, alpha);
-            }
-            if (tok < n) c[static_cast<size_t>(tok) * m + row] = __float2bfloat16(v);
+            if (tok < n) c[static_cast<size_t>(tok) * m + row] = __float2bfloat16(__uint_as_float(r[j]) * alpha);
           }
         }
       }
@@ -503,6 +544,9 @@ nvfp4_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(C::kTmemCols) : "memory");
   }
+  if (ONE && *any_odd != 0u)
+    for (uint32_t tile = blockIdx.x, t_local = 0; tile < tiles; tile += gridDim.x, ++t_local)
+      redo_rows(reinterpret_cast<const uint32_t *>(odd_rows + (t_local & 31u)), a_fp4, a_sf, b_fp4, b_sf, c, tile * kBM, k, alpha);
 }
 
 // ============================================================================================
@@ -1204,7 +1248,8 @@ nvfp4_gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   uint64_t *sf_full = empty + 8;
   uint64_t *acc_full = sf_full + 8;
   uint32_t *tmem_base_slot = reinterpret_cast<uint32_t *>(acc_full + 2);
-  volatile uint32_t *scanned = reinterpret_cast<volatile uint32_t *>(smem + 512);      // one token: 1 = the scale bytes have been looked through, 3 = and some are odd
+  uint32_t *odd_all = reinterpret_cast<uint32_t *>(smem + 384);          // one token, first CTA: [4] the rows to redo,
+  uint32_t *odd_rows = reinterpret_cast<uint32_t *>(smem + 512);         // [S][4] and what each CTA of the cluster found
   uint8_t *stages = smem + 1024;
   float *partials = reinterpret_cast<float *>(stages + C::kStages * C::kStageBytes);   // [S-1][128 rows][kCols], first CTA only
 
@@ -1221,7 +1266,6 @@ nvfp4_gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 
   if (threadIdx.x == 0) {
     for (uint32_t s = 0; s < C::kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], ONE ? 2 : 1); mbar_init(&sf_full[s], 1); }
-    *scanned = 0u;
     mbar_init(&acc_full[0], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -1308,17 +1352,19 @@ nvfp4_gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     }
   } else if (ONE && warp == kWarpScan) {
     {
-      uint32_t seen = 0u;
+      uint32_t rows[4] = {0u, 0u, 0u, 0u}, token = 0u;
       for (uint32_t kb = kb_begin, g = 0; kb < kb_end; ++kb, ++g) {
         const uint32_t s = g % C::kStages, ph = (g / C::kStages) & 1u;
         if (!mbar_wait_warp(&full[s], ph)) break;
         const uint8_t *sfa = stages + s * C::kStageBytes + C::kABytes + C::kBBytes;
-        seen |= odd_scale_bytes(sfa, sfa + C::kSfaBytes, lane);
+        scan_scale_bytes(sfa, sfa + C::kSfaBytes, lane, rows, token);
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[s]);
       }
-      const bool odd = __any_sync(0xffffffffu, seen != 0u);
-      if (lane == 0) *scanned = odd ? 3u : 1u;
+      const uint4 found = odd_rows_of(rows, token);
+      if (lane == 0)
+        asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(map_to_cta(smem_u32(odd_rows + rank * 4u), 0u)), "r"(found.x),
+                     "r"(found.y), "r"(found.z), "r"(found.w) : "memory");
     }
   } else if (warp >= kWarpEpilogue && warp < kWarpEpilogue + 4u) {
     // epilogue warps 4..7: drain this CTA's partial sums; ranks > 0 hand them to the first CTA
@@ -1338,7 +1384,6 @@ nvfp4_gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         }
       }
     }
-    if (ONE && (!count_wait(scanned, 1u) || *scanned != 1u)) acc[0] = __uint_as_float(0x7fc00000u);   // sends the row to exact_row
     if (rank != 0u) {
       const uint32_t row = quarter * 32u + lane;
       const uint32_t dst = map_to_cta(smem_u32(partials + (static_cast<size_t>(rank - 1u) * kBM + row) * kCols), 0u);
@@ -1363,15 +1408,22 @@ nvfp4_gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       }
     }
 #pragma unroll
-    for (uint32_t j = 0; j < kCols; ++j) {
-      float v = acc[j] * alpha;
-      if (ONE && j == 0u && v != v) v = exact_row(a_fp4, a_sf, b_fp4, b_sf, row, k, alpha);
-      if (j < n) c[static_cast<size_t>(j) * m + row] = __float2bfloat16(v);
-    }
+    for (uint32_t j = 0; j < kCols; ++j)
+      if (j < n) c[static_cast<size_t>(j) * m + row] = __float2bfloat16(acc[j] * alpha);
   }
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(C::kTmemCols) : "memory");
+  }
+  if (ONE && rank == 0u) {                                               // what was found is settled since the cluster met
+    uint32_t found = lane < 4u * S ? odd_rows[lane] : 0u;
+    if (__any_sync(0xffffffffu, found != 0u)) {                          // the same in every warp
+#pragma unroll
+      for (int off = 4; off < 32; off <<= 1) found |= __shfl_xor_sync(0xffffffffu, found, off);
+      if (threadIdx.x < 4u) odd_all[threadIdx.x] = found;
+      __syncthreads();
+      redo_rows(odd_all, a_fp4, a_sf, b_fp4, b_sf, c, mb * kBM, k, alpha);
+    }
   }
 }
 

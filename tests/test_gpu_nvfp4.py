@@ -496,6 +496,81 @@ def test_w4a4_one_token_every_scale_byte(backend, m, k):
     assert backend.lib.qwen36_nvfp4_gemm_last_error() == 0
 
 
+@pytest.mark.parametrize("m,k", [(12288, 3072), (5120, 6144)])
+def test_w4a4_one_token_redoes_only_the_rows_with_an_odd_scale(backend, m, k):
+    """One token on the block-scaled MMA (one tile a CTA; clusters of three along K): one scale byte of a row whose sign or whose
+    0x7F the hardware reads differently, at each of the four tiles of a stage, in the first, a middle and the last K-block (so in
+    each CTA of a cluster), in the first and the last row of a block.  The byte outweighs the rest of its row.  All other rows
+    keep their bits; so does every row when the byte is minus zero.  Rows next to the odd ones are made to cancel, so that
+    another order of summation could not give the same bits: the second half of K is minus the first."""
+    rng = np.random.default_rng(m)
+    groups = k // 16
+    packed = rng.integers(0, 256, size=(m, k // 2), dtype=np.uint8)
+    sf_rm = rng.integers(synth.SF_CODE_LO, synth.SF_CODE_HI + 1, size=(m, groups), dtype=np.uint8)
+    packed[:, k // 4:] = packed[:, : k // 4] ^ 0x88
+    sf_rm[:, groups // 2:] = sf_rm[:, : groups // 2]
+    b, b_sf, ts = orc.nvfp4_quantize_rows(np.tile(synth.activations(rng, 1, k // 2), 2), 0.4)
+    places = [(blk * 128 + r, g) for blk, (r, g) in enumerate(
+        (r, 16 * kb + i) for kb in (0, groups // 32, groups // 16 - 1) for r, i in ((0, 0), (33, 5), (70, 10), (127, 15)))]
+
+    def product(sf, alpha=0.01 * ts):
+        return bf16_host(backend.nvfp4_gemm(to_dev(packed), to_dev(orc.retile_scales(sf)), to_dev(b), to_dev(b_sf), alpha, m, 1, k))[0]
+
+    plain = product(sf_rm)
+    rows = np.array([r for r, _ in places])
+    others = np.setdiff1d(np.arange(m), rows)
+    assert np.count_nonzero(synth.bf16_bits_to_f32(plain)) > m // 8            # what cancels leaves the rounding of its sum
+    for r, g in places:                                                        # no cancelling inside the group
+        packed[r, g * 8:g * 8 + 8] = 0x77 | (b[0, g * 8:g * 8 + 8] & 0x88)
+    for byte in (0xFE, 0x7F, 0xFF):
+        sf = sf_rm.copy()
+        sf[rows, [g for _, g in places]] = byte
+        want = synth.bf16_bits_to_f32(orc.nvfp4_gemm(packed, orc.retile_scales(sf), b, b_sf, 0.01 * ts, m, 1, k))[0]
+        bits = product(sf)
+        got = synth.bf16_bits_to_f32(bits)
+        # float32 sums on either side of a bf16 rounding boundary: one unit in the last place, 2^-7 at most
+        assert np.all(np.abs(got[rows] - want[rows]) <= 2.0 ** -7 * np.abs(want[rows])) and np.all(want[rows] != 0), byte
+        assert np.array_equal(bits[others], plain[others]), byte
+    zero = sf_rm.copy()
+    zero[rows, [g for _, g in places]] = 0
+    bits = product(zero)
+    zero[rows, [g for _, g in places]] = 0x80
+    assert np.array_equal(product(zero), bits) and np.array_equal(bits[others], plain[others])
+    assert np.all(np.isnan(synth.bf16_bits_to_f32(product(sf_rm, float("nan")))))
+    assert backend.lib.qwen36_nvfp4_gemm_last_error() == 0
+
+
+@pytest.mark.parametrize("m,k", [(12288, 3072), (5120, 6144), (1024, 5120)])
+@pytest.mark.parametrize("byte", [0xFE, 0x7F, 0xFF, 0x80])
+def test_w4a4_one_token_odd_scale_of_the_token(backend, m, k, byte):
+    """A scale byte of the activation whose sign or 0x7F counts, in each tile of a stage in turn: the tiles, the clusters, the GEMV."""
+    rng = np.random.default_rng(m + byte)
+    a, a_sf, x, b, b_sf, alpha = w4a4_case(rng, m, 1, k)
+    for group in (0, 21, k // 32 + 10, k // 16 - 1):
+        odd = b_sf.copy()
+        odd[(group // 4) * 512 + group % 4] = byte
+        want = synth.bf16_bits_to_f32(orc.nvfp4_gemm(a, a_sf, b, odd, alpha, m, 1, k))
+        got = synth.bf16_bits_to_f32(bf16_host(backend.nvfp4_gemm(to_dev(a), to_dev(a_sf), to_dev(b), to_dev(odd), alpha, m, 1, k)))
+        assert rel_l2(got, want) <= 3e-3, group
+    assert backend.lib.qwen36_nvfp4_gemm_last_error() == 0 and backend.lib.qwen36_nvfp4_gemv_mma_last_error() == 0
+
+
+def test_w4a4_one_token_odd_scales_of_more_tiles_than_are_noted_apart(backend):
+    """More than 32 tiles for every CTA: the rows noted for tiles 32 apart join, and each is redone in both tiles."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    m, k = 128 * (33 * sms + 5), 256
+    rng = np.random.default_rng(5)
+    a, a_sf, x, b, b_sf, alpha = w4a4_case(rng, m, 1, k)
+    blocks = (0, 7, 20 * sms + 3, 32 * sms, 33 * sms + 4)
+    for i, blk in enumerate(blocks):
+        a_sf[blk * (k // 64) * 512 + (i % 4) * 512 + 5 * 16 + 2 * 4 + 1] = (0xFE, 0x7F)[i % 2]     # row 69, group 4 (i % 4) + 1
+    rows = np.array(blocks) * 128 + 69
+    want = synth.bf16_bits_to_f32(orc.nvfp4_gemm(a, a_sf, b, b_sf, alpha, m, 1, k))[0]
+    got = synth.bf16_bits_to_f32(bf16_host(backend.nvfp4_gemm(to_dev(a), to_dev(a_sf), to_dev(b), to_dev(b_sf), alpha, m, 1, k)))[0]
+    assert rel_l2(got[rows], want[rows]) <= 4e-3 and rel_l2(got, want) <= 3e-3
+    assert backend.lib.qwen36_nvfp4_gemm_last_error() == 0
+
+
 def test_w4a4_known_answer_132_and_alpha_zero(backend):
     # kernels-cuda/smoke.cu:2140-2180
     k = m = 128
