@@ -81,17 +81,22 @@ int launch_generic(const qwen36_nvfp4_gemm_spec_t *s, float alpha) {
   return q36::launch_status();
 }
 
+// One token: the faster of two kernels, and the other one where it declines.
+int one_token(const qwen36_nvfp4_gemm_spec_t *s, float alpha) {
+  if (q36::nvfp4_gemm_tc_forced()) return q36::nvfp4_gemm_tc(s, alpha);
+  const bool tiles = q36::nvfp4_gemm_tc_for_one_token(s);
+  const int rc = tiles ? q36::nvfp4_gemm_tc(s, alpha) : q36::nvfp4_gemv_mma_fp4(s, alpha);
+  if (rc != QWEN36_STATUS_NOT_IMPLEMENTED) return rc;
+  return tiles ? q36::nvfp4_gemv_mma_fp4(s, alpha) : q36::nvfp4_gemm_tc(s, alpha);
+}
+
 }  // namespace
 
 extern "C" int qwen36_nvfp4_gemm(const qwen36_nvfp4_gemm_spec_t *spec) {
   const int rc = check(spec);
   if (rc != QWEN36_STATUS_SUCCESS) return rc;
   const float alpha = spec->alpha == 0.0f ? 1.0f : spec->alpha;   // kernels-cuda/nvfp4_gemm.cu:380
-  if (spec->n == 1 && !q36::nvfp4_gemm_tc_forced() && !q36::nvfp4_gemm_tc_for_one_token(spec)) {
-    const int gv = q36::nvfp4_gemv_mma_fp4(spec, alpha);
-    if (gv != QWEN36_STATUS_NOT_IMPLEMENTED) return gv;
-  }
-  const int tc = q36::nvfp4_gemm_tc(spec, alpha);
+  const int tc = spec->n == 1 ? one_token(spec, alpha) : q36::nvfp4_gemm_tc(spec, alpha);
   if (tc != QWEN36_STATUS_NOT_IMPLEMENTED) return tc;
   return launch_generic(spec, alpha);
 }
@@ -100,11 +105,7 @@ extern "C" int qwen36_decode_nvfp4_gemv(const qwen36_nvfp4_gemm_spec_t *spec) {
   const int rc = check(spec);
   if (rc != QWEN36_STATUS_SUCCESS) return rc;
   if (spec->n > 8) return QWEN36_STATUS_NOT_IMPLEMENTED;
-  if (spec->n == 1 && !q36::nvfp4_gemm_tc_forced() && !q36::nvfp4_gemm_tc_for_one_token(spec)) {
-    const int gv = q36::nvfp4_gemv_mma_fp4(spec, spec->alpha);
-    if (gv != QWEN36_STATUS_NOT_IMPLEMENTED) return gv;
-  }
-  return q36::nvfp4_gemm_tc(spec, spec->alpha);   // NOT_IMPLEMENTED for shapes it declines
+  return spec->n == 1 ? one_token(spec, spec->alpha) : q36::nvfp4_gemm_tc(spec, spec->alpha);   // NOT_IMPLEMENTED for shapes they decline
 }
 
 extern "C" void qwen36_nvfp4_chunk_gemv_set_mtile(int mtile) { (void)mtile; }

@@ -91,3 +91,12 @@ def test_one_token_operands_off_sixteen_bytes_run_on_the_gemv(device):
                              abi.DevicePtr(0), 0, 1.0)
     launches, code = device.launches(lambda: device.lib.qwen36_nvfp4_gemm(C.byref(spec)))
     assert code == abi.SUCCESS and [name for name, _, _ in launches] == [GEMV]
+
+
+@pytest.mark.parametrize("entry", ["qwen36_nvfp4_gemm", "qwen36_decode_nvfp4_gemv"])
+@pytest.mark.parametrize("m,k", [(34816, 5120), (5120, 17408)])
+def test_one_token_runs_on_the_gemv_where_the_tiles_decline(device, m, k, entry):
+    """The two-dimensional tensor maps of the tiles are refused; those of the GEMV have five and three dimensions."""
+    device.lib.fake_refuse_2d_maps(1)
+    launches, code = device.product(m, 1, k, entry)
+    assert code == abi.SUCCESS and [name for name, _, _ in launches] == [GEMV]
