@@ -1111,7 +1111,7 @@ uint32_t pick_splits(const Args &a, size_t caller_splits, size_t ctas_per_split,
 }
 
 // How many clusters of `ctas` CTAs the device can hold at once with all of the shared memory (0: none); asked once per
-// device and size, together with the permission for sixteen.
+// device and size, together with the permission for sixteen.  No answer counts as none for this call and is not kept.
 template <int G, bool FP8>
 uint32_t one_launch_clusters(uint32_t ctas) {
   static std::mutex mu;
@@ -1138,7 +1138,7 @@ uint32_t one_launch_clusters(uint32_t ctas) {
       cfg.numAttrs = 1;
       if (cudaOccupancyMaxActiveClusters(&n, decode_one_launch_kernel<G, FP8>, &cfg) != cudaSuccess) {
         (void)cudaGetLastError();
-        n = 0;
+        return 0;
       }
     }
     count = n + 1;

@@ -1537,12 +1537,13 @@ bool make_scale_map(CUtensorMap *map, uint64_t ptr, uint64_t tiles) {
   return cached_map(key, map, build_scale_map);
 }
 
-// Clusters of `size` CTAs of `kernel` that the current device can host at once (asked once per kernel, size and device).
+// Clusters of `size` CTAs of `kernel` that the current device can host at once (asked once per kernel, size and device); -1 when the
+// device did not say, which is not kept.
 int max_active_clusters(const void *kernel, uint32_t size, const cudaLaunchConfig_t *cfg) {
   static std::mutex mu;
   static std::vector<std::tuple<const void *, uint32_t, int, int>> known;
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return -1;
   {
     std::lock_guard<std::mutex> lock(mu);
     for (const auto &e : known)
@@ -1551,7 +1552,7 @@ int max_active_clusters(const void *kernel, uint32_t size, const cudaLaunchConfi
   int v = 0;
   if (cudaOccupancyMaxActiveClusters(&v, kernel, cfg) != cudaSuccess) {
     (void)cudaGetLastError();
-    v = 0;
+    return -1;
   }
   std::lock_guard<std::mutex> lock(mu);
   known.emplace_back(kernel, size, dev, v);
@@ -1718,17 +1719,20 @@ uint32_t choose_split(const qwen36_nvfp4_gemm_spec_t *s, uint32_t *longest_run =
   }
   const void *kernel = reinterpret_cast<const void *>(nvfp4_gemm_splitk_kernel<BN, ONE>);
   if (q36::ensure_dynamic_smem(kernel, static_cast<int>(splitk_smem<BN>())) != cudaSuccess) return 1u;
+  bool asked = true;
   for (uint32_t split = 2u; split <= most; ++split) {
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[2];
     splitk_config<BN>(cfg, attr, m_blocks, split);
     const int fit = max_active_clusters(kernel, split, &cfg);
+    if (fit < 0) asked = false;
     if (fit <= 0) continue;
     const uint32_t rounds = (m_blocks + static_cast<uint32_t>(fit) - 1u) / static_cast<uint32_t>(fit);
     const uint32_t longest = rounds * ((k_blocks + split - 1u) / split);
     if (longest < least) { least = longest; best = split; }
   }
   if (longest_run != nullptr) *longest_run = least;
+  if (!asked) return best;                                               // the next call asks again
   slot.m_blocks = m_blocks; slot.k_blocks = k_blocks; slot.split = best; slot.longest = least; slot.dev = dev;
   return best;
 }

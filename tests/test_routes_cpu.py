@@ -100,3 +100,29 @@ def test_one_token_runs_on_the_gemv_where_the_tiles_decline(device, m, k, entry)
     device.lib.fake_refuse_2d_maps(1)
     launches, code = device.product(m, 1, k, entry)
     assert code == abi.SUCCESS and [name for name, _, _ in launches] == [GEMV]
+
+
+def test_a_failed_occupancy_query_is_asked_again(device):
+    """No answer from the device costs the call its clusters, not the process."""
+    want = Device(shutil.copy(device.lib._name, device.lib._name + ".fresh")).product(2048, 5, 6144)
+    assert want[0][0][0] == "nvfp4_gemm_splitk_kernel<8, false>"
+    device.lib.fake_fail_occupancy(7)                                   # two to eight CTAs a cluster
+    assert device.product(2048, 5, 6144) == ([("nvfp4_gemm_tc_kernel<8, false>", 16, 1)], abi.SUCCESS)
+    assert device.product(2048, 5, 6144) == want
+    device.lib.fake_fail_occupancy(1)
+    assert device.product(8192, 600, 5120)[0][0][0] != "nvfp4_gemm_pair6_kernel<false>"
+    assert device.product(8192, 600, 5120)[0][0][0] == "nvfp4_gemm_pair6_kernel<false>"
+
+
+def test_a_failed_occupancy_query_of_decode_attention_is_asked_again(device):
+    p = [abi.DevicePtr(BASE + (i << 34)) for i in range(9)]
+    spec = abi.AttentionDecodeSpec(0, 599, *p[:5], abi.DevicePtr(0), p[5], abi.AttentionShape(24, 4, 256, 0), 1, abi.DevicePtr(0), *p[6:], 256, 0)
+
+    def kernels():
+        launches, code = device.launches(lambda: device.lib.qwen36_attention_decode(C.byref(spec)))
+        assert code == abi.SUCCESS
+        return [re.sub("<.*", "", name) for name, _, _ in launches]
+
+    device.lib.fake_fail_occupancy(2)                                   # sixteen CTAs, eight
+    assert "decode_one_launch_kernel" not in kernels()
+    assert kernels() == ["decode_one_launch_kernel"]
