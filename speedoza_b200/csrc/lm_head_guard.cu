@@ -666,8 +666,12 @@ extern "C" int qwen36_bf16_matvec_argmax_rows(const qwen36_bf16_matvec_argmax_ro
       spec->in_features * sizeof(float) > 200 * 1024)
     return QWEN36_STATUS_INVALID_ARGUMENT;
   const unsigned blocks = static_cast<unsigned>(q36::div_ceil(spec->rows, static_cast<size_t>(128)));
-  if (q36::launch_after_previous(bf16_argmax_clear_kernel, dim3(blocks), dim3(128), size_t{0}, q36::stream(),
-                                 as_ptr<unsigned long long>(spec->workspace), static_cast<size_t>(spec->rows)) != cudaSuccess)
+  // Keys off an eight-byte boundary are never touched when every row is certified, so they are cleared as bytes.
+  const bool cleared = spec->workspace.ptr % sizeof(unsigned long long) != 0
+                           ? cudaMemsetAsync(as_ptr<void>(spec->workspace), 0, spec->rows * sizeof(unsigned long long), q36::stream()) == cudaSuccess
+                           : q36::launch_after_previous(bf16_argmax_clear_kernel, dim3(blocks), dim3(128), size_t{0}, q36::stream(),
+                                                        as_ptr<unsigned long long>(spec->workspace), static_cast<size_t>(spec->rows)) == cudaSuccess;
+  if (!cleared)
     return QWEN36_STATUS_CUDA_ERROR;
   // Rows per pass: as many as the float32 staging of their activations allows (at most eight).
   // Every pass skips flagged rows itself, so a pass over rows that are all flagged reads nothing.

@@ -126,3 +126,12 @@ def test_a_failed_occupancy_query_of_decode_attention_is_asked_again(device):
     device.lib.fake_fail_occupancy(2)                                   # sixteen CTAs, eight
     assert "decode_one_launch_kernel" not in kernels()
     assert kernels() == ["decode_one_launch_kernel"]
+
+
+@pytest.mark.parametrize("offset", [0, 4])
+def test_argmax_keys_off_their_alignment_are_cleared_as_bytes(device, offset):
+    p = [abi.DevicePtr(BASE + (i << 34)) for i in range(6)]
+    spec = abi.Bf16MatvecArgmaxRowsSpec(3, 4096, 1024, p[0], p[1], p[2], abi.DevicePtr(0), abi.DevicePtr(p[3].ptr + offset), 64, p[4])
+    launches, code = device.launches(lambda: device.lib.qwen36_bf16_matvec_argmax_rows(C.byref(spec)))
+    assert code == abi.SUCCESS
+    assert ("bf16_argmax_clear_kernel" in [name for name, _, _ in launches], device.lib.fake_memsets()) == ((True, 0) if offset == 0 else (False, 1))
