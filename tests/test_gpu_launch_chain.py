@@ -83,3 +83,73 @@ def test_feed_forward_chain_on_shared_buffers(backend, tokens):
         block(i, lambda: None)
         wrong += (out != want[i % 4]).sum()
     assert wrong.item() == 0 and out.float().abs().max().item() > 0.1
+
+
+@pytest.mark.parametrize("hidden,inter", [(3072, 6144), (2560, 4352)])
+def test_one_token_feed_forward_chain_on_shared_buffers(backend, hidden, inter):
+    """Norm + quantise, gate_up, SwiGLU + quantise, down at one token; tiles and clusters in the first case, the GEMV, which
+    reads its weights ahead of its wait, in the second."""
+    gen = torch.Generator(device="cuda").manual_seed(hidden)
+    w = [(*weight(backend, gen, 2 * inter, hidden), *weight(backend, gen, hidden, inter)) for _ in range(2)]
+    xs, residual, norm = rows(gen, 4, hidden), rows(gen, hidden), rows(gen, hidden) * 0.1
+    q = backend.rmsnorm_nvfp4_quantize(xs[0], norm, residual, 1e-6, 0.37, False, True)
+    gate_up = torch.zeros((1, 2 * inter), dtype=torch.bfloat16, device="cuda")
+    act = backend.swiglu_nvfp4_quantize(gate_up[0, :inter], gate_up[0, inter:], 0.11)
+    out = torch.empty((1, hidden), dtype=torch.bfloat16, device="cuda")
+
+    def block(i, settle):
+        w1, sf1, w2, sf2 = w[i % 2]
+        backend.rmsnorm_nvfp4_quantize(xs[i % 4], norm, residual, 1e-6, 0.37, False, True, q)
+        settle()
+        backend.nvfp4_gemm(w1, sf1, q[2], q[3], 5e-4, 2 * inter, 1, hidden, gate_up)
+        settle()
+        backend.swiglu_nvfp4_quantize(gate_up[0, :inter], gate_up[0, inter:], 0.11, *act)
+        settle()
+        backend.nvfp4_gemm(w2, sf2, act[0], act[1], 5e-4, hidden, 1, inter, out)
+        settle()
+
+    want = torch.empty((4, 1, hidden), dtype=torch.bfloat16, device="cuda")
+    for i in range(4):
+        block(i, torch.cuda.synchronize)
+        want[i] = out
+    wrong = torch.zeros((), dtype=torch.int64, device="cuda")
+    for i in range(40):
+        block(i, lambda: None)
+        wrong += (out != want[i % 4]).sum()
+    assert wrong.item() == 0 and out.float().abs().max().item() > 0.1
+    assert backend.lib.qwen36_nvfp4_gemm_last_error() == 0 and backend.lib.qwen36_nvfp4_gemv_mma_last_error() == 0
+
+
+def test_guard_and_argmax_chain_on_shared_buffers(backend):
+    """FP8 logits, top-8 guard, and the bf16 argmax of the rows it did not certify (clear, scan, result), over and over into the
+    same logits, tokens and flags; ten rows, so that the argmax scans in two passes, of which some have nothing to do."""
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    vocab, hidden, n = 20000, 1024, 10
+    wb = torch.empty((vocab, hidden), dtype=torch.bfloat16, device="cuda").normal_(0.0, 0.02, generator=gen)
+    w8, scales = backend.lm_head_fp8_quantize(wb)
+    xs = torch.randn((4, n, hidden), generator=gen, device="cuda")
+    pick = torch.randint(0, vocab, (4, n), generator=gen, device="cuda")
+    boost = torch.full((4, n, 1), 10.0, device="cuda")
+    boost[1] = 0.0                                   # no row certified, rows 2 and 9, all certified, the second pass alone
+    boost[2, [2, 9]] = 0.0
+    boost[0, 8:] = 0.0
+    xs = (xs + boost * wb[pick].float() / (0.02 * hidden ** 0.5)).to(torch.bfloat16)
+    logits = torch.empty((n, vocab), dtype=torch.bfloat16, device="cuda")
+
+    def step(i, settle):
+        backend.lm_head_fp8_gemv(w8, scales, xs[i % 4], logits)
+        settle()
+        tokens, flags = backend.lm_head_top8_rescore(logits, wb, xs[i % 4], 2.0)
+        settle()
+        backend.bf16_matvec_argmax_rows(xs[i % 4], wb, tokens, flags)
+        settle()
+        return torch.stack((tokens, flags))
+
+    want = torch.stack([step(i, torch.cuda.synchronize) for i in range(4)])
+    got = torch.stack([step(i, lambda: None) for i in range(40)])
+    torch.cuda.synchronize()
+    assert torch.equal(got, want.repeat(10, 1, 1))
+    flags = want[:, 1].ne(0)
+    assert flags[3].all() and not flags[1].any() and flags[2].sum() == 8 and flags[0, :8].all() and not flags[0, 8:].any()
+    full = torch.stack([(x.float() @ wb.float().T).argmax(1) for x in xs])
+    assert (want[:, 0] == full).float().mean() > 0.9                   # near ties of unpeaked rows aside

@@ -445,25 +445,32 @@ def test_w4a4_decode_split_k(backend, m, n, k):
 
 @pytest.mark.parametrize("m,k", [(1024, 5120), (5120, 6144), (5120, 17408), (12288, 5120), (128, 256), (384, 1280)])
 def test_w4a4_one_token_decode_vs_oracle(backend, m, k):
-    """One token through qwen36_decode_nvfp4_gemv and qwen36_nvfp4_gemm (the route of the
-    5120 x 17408 down projection): the tensor-core GEMV with the activation dequantised to float16
-    (exact).  rel-L2 <= 1e-2 against the float64 oracle (in fact ~1e-3: bf16 rounding of the output)."""
+    """One token through qwen36_decode_nvfp4_gemv and qwen36_nvfp4_gemm, by the route that the shape takes (block-scaled tiles or
+    clusters; the tensor-core GEMV with the activation dequantised to float16, exact) and with the tiles pinned.  Only the bf16
+    rounding of the output separates it from the float64 oracle."""
     rng = np.random.default_rng(m + k)
     a, a_sf, x, b, b_sf, alpha = w4a4_case(rng, m, 1, k)
     want = synth.bf16_bits_to_f32(orc.nvfp4_gemm(a, a_sf, b, b_sf, alpha, m, 1, k))
     dev = [to_dev(t) for t in (a, a_sf, b, b_sf)]
-    for entry in (backend.decode_nvfp4_gemv_raw, backend.nvfp4_gemm_raw):
-        out = torch.full((1, m), float("nan"), dtype=torch.bfloat16, device="cuda")
-        assert entry(*dev, alpha, m, 1, k, out) == abi.SUCCESS
-        got = synth.bf16_bits_to_f32(bf16_host(out))
-        assert rel_l2(got, want) <= 3e-3
-    assert backend.lib.qwen36_nvfp4_gemv_mma_last_error() == 0
+    try:
+        for pinned in (0, 8):
+            backend.lib.qwen36_nvfp4_gemm_force_bn(pinned)
+            for entry in (backend.decode_nvfp4_gemv_raw, backend.nvfp4_gemm_raw):
+                out = torch.full((1, m), float("nan"), dtype=torch.bfloat16, device="cuda")
+                assert entry(*dev, alpha, m, 1, k, out) == abi.SUCCESS
+                got = synth.bf16_bits_to_f32(bf16_host(out))
+                assert rel_l2(got, want) <= 3e-3
+    finally:
+        backend.lib.qwen36_nvfp4_gemm_force_bn(0)
+    assert backend.lib.qwen36_nvfp4_gemv_mma_last_error() == 0 and backend.lib.qwen36_nvfp4_gemm_last_error() == 0
 
 
-@pytest.mark.parametrize("m,k,n", [(2048, 1536, 5), (3584, 3072, 2), (4608, 2048, 16), (2048, 4096, 32), (1024, 3072, 8), (5120, 12288, 40)])
+@pytest.mark.parametrize("m,k,n", [(2048, 1536, 5), (2048, 4352, 8), (2048, 6144, 16), (3584, 3072, 2), (4608, 2048, 16), (2048, 4096, 32),
+                                   (1024, 3072, 8), (5120, 12288, 40)])
 def test_w4a4_split_k_with_as_many_ctas_as_have_room_together(backend, m, k, n):
-    """Row-block counts at which SMs / row blocks would give clusters that do not fit the GPU all at once (16 of eight CTAs, 28 of
-    five, 36 of four), and two that keep their split.  Only the bf16 rounding of the output (2^-9) separates it from the oracle."""
+    """The results at row-block counts where SMs / row blocks would give clusters that do not fit the GPU all at once (16 of
+    eight CTAs at 17 and 24 K-blocks, 28 of five, 36 of four), and at some that keep their split; test_routes_cpu.py has the choice
+    itself.  Only the bf16 rounding of the output (2^-9) separates it from the oracle."""
     rng = np.random.default_rng(m + k + n)
     a, a_sf, x, b, b_sf, alpha = w4a4_case(rng, m, n, k)
     want = synth.bf16_bits_to_f32(orc.nvfp4_gemm(a, a_sf, b, b_sf, alpha, m, n, k))
@@ -472,10 +479,11 @@ def test_w4a4_split_k_with_as_many_ctas_as_have_room_together(backend, m, k, n):
     assert backend.lib.qwen36_nvfp4_gemm_last_error() == 0
 
 
-@pytest.mark.parametrize("m,k", [(12288, 256), (5120, 1536), (37632, 512), (11904, 256)])
+@pytest.mark.parametrize("m,k", [(12288, 256), (5120, 1536), (5120, 4096), (37632, 512), (11904, 256), (22016, 5120), (1024, 5120)])
 def test_w4a4_one_token_every_scale_byte(backend, m, k):
-    """One token where the block-scaled MMA takes it (one tile a CTA, clusters along K, two rounds) and where the GEMV does: all
-    256 scale bytes among the weights of some row blocks, whose signs and 0x7F the reference honours, ordinary ones elsewhere."""
+    """One token where the block-scaled MMA takes it (one tile a CTA, clusters along K in the third case, two rounds in the fourth)
+    and where the GEMV does (5120 x 1536, 22016 x 5120, 1024 x 5120): all 256 scale bytes among the weights of some row blocks, whose
+    signs and 0x7F the reference honours, ordinary ones elsewhere."""
     rng = np.random.default_rng(m + k)
     packed = rng.integers(0, 256, size=(m, k // 2), dtype=np.uint8)
     sf_rm = rng.integers(synth.SF_CODE_LO, synth.SF_CODE_HI + 1, size=(m, k // 16), dtype=np.uint8)
@@ -493,7 +501,7 @@ def test_w4a4_one_token_every_scale_byte(backend, m, k):
     assert np.isfinite(got).all() and rel_l2(got, want) <= 3e-3
     plain = np.setdiff1d(np.arange(m), (odd[:, None] * 128 + np.arange(128)).ravel())
     assert rel_l2(got[:, plain], want[:, plain]) <= 3e-3
-    assert backend.lib.qwen36_nvfp4_gemm_last_error() == 0
+    assert backend.lib.qwen36_nvfp4_gemm_last_error() == 0 and backend.lib.qwen36_nvfp4_gemv_mma_last_error() == 0
 
 
 @pytest.mark.parametrize("m,k", [(12288, 3072), (5120, 6144)])

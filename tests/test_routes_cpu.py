@@ -102,6 +102,30 @@ def test_one_token_runs_on_the_gemv_where_the_tiles_decline(device, m, k, entry)
     assert code == abi.SUCCESS and [name for name, _, _ in launches] == [GEMV]
 
 
+def split_choice(device, m_blocks, k_blocks, at_most):
+    """CTAs per row block: the longest CTA's K-blocks over all rounds are fewest, the smaller of equals; 1 = no clusters."""
+    best, least = 1, k_blocks * -(-m_blocks // 148)
+    for split in range(2, min(148 // m_blocks, at_most, k_blocks // 2) + 1):
+        longest = -(-m_blocks // device.lib.fake_clusters(split)) * -(-k_blocks // split)
+        if longest < least:
+            best, least = split, longest
+    return best
+
+
+def test_split_k_clusters_are_as_large_as_fit_one_per_row_block(device):
+    """Every row-block count that can be split, over K-block counts that meet in the same slots of the table of known choices
+    ((31 row blocks + 7 K-blocks) mod 64); asked twice, the second time in another order."""
+    shapes = [(mb, kb) for mb in range(1, 76) for kb in (4, 16, 24, 68, 80, 88)]
+    tables = (2, "nvfp4_gemm_{}_kernel<8, false>", 8), (9, "nvfp4_gemm_{}_kernel<16, false>", 8), (17, "nvfp4_gemm_{}_kernel<32, false>", 5)
+    for tokens, kernel, at_most in tables:
+        for mb, kb in shapes + shapes[::-7] + shapes[::-3]:
+            split = split_choice(device, mb, kb, at_most)
+            want = (kernel.format("splitk"), mb * split, split) if split > 1 else (kernel.format("tc"), mb, 1)
+            assert device.product(128 * mb, tokens, 256 * kb) == ([want], abi.SUCCESS), (mb, kb)
+    # 16 row blocks, where clusters of eight have room for 15 only, and 36, where those of four have room for 34
+    assert [split_choice(device, mb, 24, 8) for mb in (15, 16, 28, 36)] == [8, 6, 4, 3]
+
+
 def test_a_failed_occupancy_query_is_asked_again(device):
     """No answer from the device costs the call its clusters, not the process."""
     want = Device(shutil.copy(device.lib._name, device.lib._name + ".fresh")).product(2048, 5, 6144)
