@@ -1783,10 +1783,10 @@ bool nvfp4_gemm_tc_forced() { return g_force_bn.load() != 0 || g_force_split.loa
 //  * Tiles, one per CTA: from 0.62 (12288 x 5120 13.0 11.2, 13.3 12.6, 12.7 10.9; 18944 x 4096 12.6 11.4, 12.9 12.6, 12.1 11.2); short K from
 //    0.70 (12288 x 2048, 0.65: 8.1 7.2, but 8.4 8.5 and 6.9 7.1).  The GEMV goes through K in steps of 1024, so other K count as the next
 //    multiple: eight blocks of 2304 x 6144 take 129.8 us with tiles for gate_up, 135.7 with the GEMV; of 2048 x 6144 126.5 and 123.6.
-//  * More rounds of tiles (the GEMV has none): from 0.72 for two (28672 x 5120 20.8 18.7, 21.9 20.1, 20.8 18.5; 24576 x 4096, 0.65: 15.3
+//  * More rounds of tiles (the GEMV has none): from 0.71 for two (28672 x 5120 20.8 18.7, 21.9 20.1, 20.8 18.5; 24576 x 4096, 0.65: 15.3
 //    15.9, 15.8 17.0, 15.8 15.4), 0.78 for more (44800 x 5120, 0.79: 28.6 26.7, 29.5 28.5, 28.2 26.5; 57344 x 4096, 0.76: 27.2 28.4); shorter
-//    K sooner, from 0.69 below 4096 and 0.62 below 3072 (eight blocks: 3072 x 11776, 0.62, 184.6 us with the GEMV for gate_up, 187.6 with
-//    tiles; 3584 x 11264, 0.68, 196.3 199.9; 3072 x 13824, 0.73, 203.5 190.7; 2048 x 11776, 0.62, 165.4 161.5).
+//    K sooner, from 0.64 below 4096 and 0.62 below 3072 (eight blocks: 3072 x 11776, 0.62, 183.8 us with the GEMV for gate_up, 186.6 with
+//    tiles; 3072 x 12800, 0.68, 194.3 185.9; 3584 x 11264, 0.68, 196.9 194.6; 2048 x 11776, 0.62, 165.4 161.5).
 //  * Clusters: from 0.60 (2048 x 17408, 0.61: 11.8 9.3).  They cost 0.6 us more than one CTA per tile, so K has to be long: from 3584
 //    where every SM has more than one of the GEMV's units (5632 x 3584 7.3 6.8, 8.3 7.7, 7.1 6.9; x 2048 5.5 5.8), from 6144 where it has
 //    one at most (3072 x 6656 8.5 7.1, 9.9 8.6, 8.6 7.1; x 6144 7.0 6.9, 8.5 8.4, 6.7 7.0; x 5120 6.3 6.6, 7.9 7.9, 6.2 6.6), above 8192 where
@@ -1805,7 +1805,7 @@ bool nvfp4_gemm_tc_for_one_token(const qwen36_nvfp4_gemm_spec_t *s) {
     least = 60u;
   } else {
     k_blocks = static_cast<uint32_t>(q36::round_up(k_blocks, 4));
-    least = rounds == 1u ? (k < 3072u ? 70u : 62u) : k < 3072u ? 62u : k < 4096u ? 69u : rounds == 2u ? 72u : 78u;
+    least = rounds == 1u ? (k < 3072u ? 70u : 62u) : k < 3072u ? 62u : k < 4096u ? 64u : rounds == 2u ? 71u : 78u;
   }
   return static_cast<uint64_t>(m_blocks) * k_blocks * 100u >= static_cast<uint64_t>(sms) * longest * least;
 }
