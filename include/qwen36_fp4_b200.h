@@ -246,10 +246,14 @@ int qwen36_swiglu_nvfp4_quantize_rows(const qwen36_swiglu_nvfp4_quantize_rows_sp
 /* Replaces qwen36_nvfp4_gemm (kernels-cuda/nvfp4_gemm.cu:341-409, a cuBLASLt
  * call).  Any m, n, k with k % 16 == 0.  alpha == 0 is read as 1.  Shapes with
  * m % 128 == 0 and k % 256 == 0 run on tcgen05 block-scaled MMA: persistent
- * 128-row x {8..256}-token tiles; for n <= 16 with fewer row blocks than SMs,
- * clusters of CTAs split K and add their partial sums through distributed
- * shared memory; for long K and thousands of tokens, CTA pairs (cta_group::2)
- * share 256 x 256 tiles.  Anything else takes a generic SIMT kernel. */
+ * 128-row x {8..256}-token tiles; for n <= 64 with few row blocks, clusters of
+ * CTAs split K and add their partial sums through distributed shared memory;
+ * from 512 tokens up CTA pairs (cta_group::2) share 256 x 256 tiles.  One token
+ * takes those tiles or the one-token GEMV, whichever measured faster at its
+ * shape.  Anything else takes a generic SIMT kernel.  At one token every scale
+ * byte is read as the reference's scalar kernels read it (sign honoured,
+ * 0x7F = 448); two tokens and more on the block-scaled MMA take 0x00 .. 0x7E,
+ * which is what the quantisers write. */
 int qwen36_nvfp4_gemm(const qwen36_nvfp4_gemm_spec_t *spec);
 
 /* Replaces qwen36_decode_nvfp4_gemv
@@ -264,9 +268,10 @@ int qwen36_decode_nvfp4_gemv(const qwen36_nvfp4_gemm_spec_t *spec);
 void qwen36_nvfp4_chunk_gemv_set_mtile(int mtile);
 
 /* Replaces qwen36_nvfp4_matvec (kernels-cuda/ops.cu:547-639,1155-1180).  The
- * one-token kernels (this one, its group form, qwen36_decode_nvfp4_gemv and
- * qwen36_nvfp4_gemm at n = 1) start while the call ahead on the stream drains
- * and read weights, scales and tensor scale before they wait for it.  What this
+ * one-token GEMVs (this one, its group form, and qwen36_decode_nvfp4_gemv and
+ * qwen36_nvfp4_gemm at n = 1 for the shapes that they take by GEMV) start while
+ * the call ahead on the stream drains and read weights, scales and tensor scale
+ * before they wait for it; the tiles read nothing before they wait.  What this
  * library's quantisers write is complete by then; another kernel of this
  * library that writes a weight must not be the call directly ahead. */
 int qwen36_nvfp4_matvec(const qwen36_nvfp4_matvec_spec_t *spec);

@@ -1150,10 +1150,10 @@ uint32_t one_launch_clusters(uint32_t ctas) {
 // context on the host (its shared memory is sized by it), all of it in one cluster's shared memory, and a cluster per kv
 // head on the device at the same time: there it is the faster one throughout, in two rounds it is not.  us per layer,
 // graph replay, split + merge | cluster of 8 | of 16 (-: does not fit; eight CTAs hold half the rows):
-//   24 / 4 heads, FP8    64 rows 7.2 | 4.6 | 4.8    400  9.5 | 5.0 | 5.1   1000  9.5 | 5.8 | 5.5   3000 10.4 | 9.6 |  7.7   5000 11.1 |  -  |  9.5
-//                 BF16   64 rows 6.9 | 4.2 | 4.4    400 10.9 | 4.9 | 4.9   1000 11.6 | 6.0 | 5.5   2000 11.8 |  -  |  7.4   3000 12.1 |  -  |  8.7
-//   32 / 8 heads, FP8    64 rows 6.7 | 4.5 | 8.7    400  9.0 | 5.0 | 9.4   1000  9.0 | 5.8 | 10.1  3000 10.9 | 10.0 | 14.8  5000 13.7 |  -  | 18.3
-//   64 / 16 heads, FP8   64 rows 6.7 | 8.3 | 13.0   400  9.0 | 9.1 | 14.0  1000 10.4 | 12.6 | 17.7
+//   24 / 4 heads, FP8    64 rows 6.8 | 4.5 | 4.8    400  9.1 | 4.9 | 5.1   1000  9.4 | 5.8 | 5.5   3000 10.2 | 9.4 |  7.4   5000 10.7 |  -  |  9.2
+//                 BF16   64 rows 6.6 | 4.1 | 4.4    400 10.6 | 4.9 | 4.9   1000 11.1 | 5.9 | 5.4   2000 11.5 |  -  |  7.2   3000 11.6 |  -  |  8.4
+//   32 / 8 heads, FP8    64 rows 6.4 | 4.5 | 8.7    400  8.8 | 4.9 | 9.4   1000  9.1 | 5.8 | 10.1  3000 10.4 |  9.8 | 14.3  5000 13.3 |  -  | 18.1
+//   64 / 16 heads, FP8   64 rows 6.6 | 8.1 | 13.2   400  8.9 | 9.0 | 14.2  1000 10.4 | 11.8 | 16.9
 // (a B200 holds six or seven clusters of sixteen, twelve to fifteen of eight)
 // Between the cluster sizes the line lies at 512 rows.
 template <int G, bool FP8>

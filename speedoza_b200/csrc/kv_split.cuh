@@ -14,9 +14,10 @@ namespace q36 {
 constexpr int kSplitThreads = 256;
 constexpr int kSplitWarps = kSplitThreads / 32;
 // Tokens of a split that L2 is asked for before the wait, in launches of kAheadFrom splits and more.  128 is the first stage of every warp;
-// 4 KB a request (a request per cache row cost more than it gave).  us a layer without | 128 tokens | 256: int8 4097 rows 12.69 | 12.50 |
-// 12.31, 16384 17.9 | 17.3 | 17.6, 131072 52.6 | 52.2 | 52.7; FP8 10000 14.1 | 13.7 | 13.9, 65536 29.5 | 28.9 | 29.8; BF16 5000 12.6 | 11.9 | 12.1.
-// Three splits (600 rows) lost 0.07 us by it.
+// 4 KB a request (a request per cache row cost more than it gave).  us a layer without | with, replayed in turn on one device: int8
+// 4097 rows 12.93 | 12.74, 16384 18.1 | 17.5, 131072 56.0 | 55.5; FP8 10000 14.10 | 13.58, 65536 29.2 | 28.6; BF16 5000 12.72 | 11.94.  256
+// tokens were 0.2 us better at 4097 rows and 0.2 - 0.9 worse from 10000 on; three splits (600 rows) lost 0.07 us by it.  The lines
+// that ask stand in each kernel: as one function in this file they cost int8 131072 0.5 us a layer.
 constexpr uint32_t kSplitAhead = 128, kAheadFrom = 8;
 
 __device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,

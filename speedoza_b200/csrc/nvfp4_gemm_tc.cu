@@ -1693,7 +1693,8 @@ void splitk_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute (&attr)[2], uint
 // that makes the longest CTA's K-blocks, over all rounds, fewest, the smaller of equals.  A cluster's CTAs share a GPC of
 // 16 to 20 SMs, so far fewer clusters fit than SMs / split: sixteen clusters of eight ran as two rounds, and so did 28 of five and
 // 36 of four.  One token, us, with SMs / row blocks as the rule | with this one: 2048 x 6144 8.2 | 4.7, 3584 x 12288 12.7 | 7.7,
-// 4608 x 16384 17.0 | 10.8; 5120 rows keep their three.
+// 4608 x 16384 17.0 | 10.8; 5120 rows keep their three.  Behind the row quantiser: 2048 x 6144 2, 9 and 16 tokens 10.6 | 6.6, 13.2 | 7.8,
+// 13.5 | 8.1; 3584 x 12288 at 17 and 32 tokens 20.7 | 13.9, 21.1 | 14.1; 33 and 64 tokens are as before.
 template <uint32_t BN, bool ONE = false>
 uint32_t choose_split(const qwen36_nvfp4_gemm_spec_t *s, uint32_t *longest_run = nullptr) {
   const uint32_t m_blocks = static_cast<uint32_t>(s->m / kBM), k_blocks = static_cast<uint32_t>(s->k / 256);
