@@ -119,6 +119,36 @@ def test_bf16_matvec_argmax_rows_vs_oracle(backend, rows, vocab, cols):
     assert mirror.item() == (-5 if skip[rows - 1] else int(want[rows - 1]))
 
 
+@pytest.mark.parametrize("captured", [False, True])
+def test_bf16_matvec_argmax_rows_keys_off_their_alignment(backend, captured):
+    """A workspace at four bytes past an eight-byte boundary, every row certified: nothing touches the keys, the tokens stay."""
+    rng = np.random.default_rng(8)
+    rows, vocab, cols = 3, 2000, 512
+    w, x, _ = make_head(rng, vocab, cols, rows, 0.0)
+    wd, xd = to_dev(w), to_dev(x)
+    tokens, mirror = (torch.arange(7, 7 + n, dtype=torch.int32, device="cuda") for n in (rows, 1))
+    flags = torch.ones(rows, dtype=torch.int32, device="cuda")
+    ws = torch.full((8 * rows + 8,), 0x55, dtype=torch.uint8, device="cuda")
+    spec = abi.Bf16MatvecArgmaxRowsSpec(rows, vocab, cols, dp(xd), dp(wd), dp(tokens), dp(mirror), abi.DevicePtr(ws.data_ptr() + 4), 8 * rows,
+                                        dp(flags))
+
+    def call():
+        assert backend.lib.qwen36_bf16_matvec_argmax_rows(C.byref(spec)) == abi.SUCCESS
+
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            backend.sync_stream()
+            call()
+        backend.sync_stream()
+        graph.replay()
+    else:
+        call()
+    torch.cuda.synchronize()
+    assert tokens.tolist() == [7, 8, 9] and mirror.item() == 7
+    assert ws.tolist() == [0x55] * 4 + [0] * (8 * rows) + [0x55] * 4
+
+
 def test_two_stage_pipeline_equals_full_bf16_argmax(backend):
     """Stage 1 (guard over FP8-like logits) + stage 2 (predicated bf16 rescore of the failed rows)
     gives the bf16 argmax for every row."""
